@@ -15,8 +15,8 @@
 // take turns.  A page-sized tile is 72 KB; with Q_eff out of shared memory the ring holds three
 // tiles, so the copies of the next tiles are in flight while this one is computed.
 //
-// MMA issue.  One thread issues a tcgen05.mma about every 50-80 cycles whatever its size, and a
-// 64-token tile needs 36 QK MMAs (K = 16 each) and 8 SV MMAs: there are two QK issuers (each
+// MMA issue.  A 64-token tile needs 36 QK MMAs (K = 16 each) and 8 SV MMAs, and every barrier wait in
+// between costs an issuer a few hundred cycles: there are two QK issuers (each
 // accumulates half of the chunks of every tile into a score buffer of its own) and one SV issuer.
 // They touch different accumulators and are ordered against each other only through the mbarriers
 // of the softmax hand-off.
@@ -255,23 +255,38 @@ __device__ __forceinline__ void finish_token(const StreamParams& p, int tok, int
   }
 }
 
+// A barrier wait of a whole warp: all lanes go on, or none.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* d_status, int code) {
+  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, abort_flag, d_status, code));
+}
+
 // The QK MMAs of chunks [C0, C1) of tile g: S_partial = Q[:, chunks] * K[:, chunks]^T.  Chunks land
-// in groups of three, each group with a barrier.
+// in groups of three, each group with a barrier; the next group's is asked before this group's MMAs
+// are issued (the answer takes longer than the issue).  Whole warp; one elected lane issues.
 template <int C0, int C1>
 __device__ __forceinline__ bool qk_chunks(StreamMisc* mi, int g, uint32_t d, uint32_t tmem, uint32_t frame16,
                                           volatile int* abort_flag, int* d_status) {
   constexpr uint32_t idesc_qk = tc::umma_idesc_bf16(HEADS, TILE, 0, 0);
   const uint64_t k_major = tc::umma_desc_sw128(0, 16, 1024);
+  const uint32_t parity = (g >> 2) & 1;
+  bool ready = tc::mbar_try_wait(&mi->full_t[g & 3][C0 / 3], parity);
 #pragma unroll
-  for (int c = C0; c < C1; ++c) {
-    if (c == C0 || c % 3 == 0) {
-      if (!tc::mbar_wait(&mi->full_t[g & 3][c / 3], (g >> 2) & 1, abort_flag, d_status, ST_MMA_TIMEOUT)) return false;
-      tc::tc_fence_after();
+  for (int c0 = C0; c0 < C1; c0 = (c0 / 3 + 1) * 3) {
+    if (!__all_sync(0xffffffffu, ready) &&
+        !warp_wait(&mi->full_t[g & 3][c0 / 3], parity, abort_flag, d_status, ST_MMA_TIMEOUT))
+      return false;
+    const int c_next = (c0 / 3 + 1) * 3;
+    if (c_next < C1) ready = tc::mbar_test_wait(&mi->full_t[g & 3][c_next / 3], parity);
+    if (tc::elect_one()) {
+#pragma unroll
+      for (int c = c0; c < c_next && c < C1; ++c) {
+        const uint64_t db = k_major | (uint64_t)(frame16 + c * (CHUNK / 16));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_ts(d, tmem + COL_Q + c * 32 + k * 8, db + k * 2, idesc_qk, (c > C0 || k > 0) ? 1u : 0u);
+      }
     }
-    const uint64_t db = k_major | (uint64_t)(frame16 + c * (CHUNK / 16));
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      umma_ts(d, tmem + COL_Q + c * 32 + k * 8, db + k * 2, idesc_qk, (c > C0 || k > 0) ? 1u : 0u);
+    __syncwarp();
   }
   return true;
 }
@@ -363,11 +378,12 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
     }
   } else if (warp == 1 || warp == 13) {
     // ---------------- QK issuers ----------------
-    // A thread issues a tcgen05.mma about every 50-80 cycles, whatever its size, and needs a few
-    // hundred cycles per barrier it waits on, so the 36 QK MMAs of a tile are split: warp 1
-    // accumulates chunks 0-4 and warp 13 chunks 5-8 into score buffers of their own (the
-    // softmax threads add the two).  Partial k = 2g + part lives in buffer k % 3.
-    if (lane == 0) {
+    // A thread needs a few hundred cycles per barrier it waits on and 30 per MMA, so the 36 QK MMAs of a
+    // tile are split: warp 1 accumulates chunks 0-4 and warp 13 chunks 5-8 into score buffers of
+    // their own (the softmax threads add the two).  Partial k = 2g + part lives in buffer k % 3.
+    // The whole warp walks the tiles and one elected lane issues: warp-uniform control flow keeps the
+    // descriptors in uniform registers (from a lane-0 branch an MMA took 65 cycles to issue).
+    {
       const int part = warp == 1 ? 0 : 1;
       const uint32_t ring16 = (tc::smem_u32(s_ring) & 0x3FFFFu) >> 4;
       TileCursor cur;
@@ -378,8 +394,8 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
         // both issuers wait for Q_eff of every segment; all softmax threads have read the block's
         // frame by then, which is what the producers wait for before they reuse it
         if (cur.t == 0) {
-          ok = tc::mbar_wait(&mi->q_ready, cur.sidx & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
-          if (ok && part == 0) tc::mbar_arrive(&mi->o_done[cur.gq & 3]);
+          ok = warp_wait(&mi->q_ready, cur.sidx & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
+          if (ok && part == 0 && lane == 0) tc::mbar_arrive(&mi->o_done[cur.gq & 3]);
         }
         if (WHOLE && (n & 1) != part) {  // the other issuer's tile
           cur.next(p.segs);
@@ -387,44 +403,47 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
         }
         const int k = WHOLE ? n : 2 * n + part, buf = k % 3, use = k / 3;
         // the softmax threads have read the previous partial in this buffer
-        if (ok && use >= 1) ok = tc::mbar_wait(&mi->s_free[buf], (use - 1) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
+        if (ok && use >= 1) ok = warp_wait(&mi->s_free[buf], (use - 1) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
         if (!ok) break;
+        tc::tc_fence_after();
         const uint32_t d = tmem + COL_S + buf * TILE;  // same lanes as the TMEM-resident A
         const uint32_t frame16 = ring16 + (g % 3) * NCH * (CHUNK / 16);
         if (WHOLE) ok = qk_chunks<0, NCH>(mi, g, d, tmem, frame16, abort_flag, p.d_status);
         else if (part == 0) ok = qk_chunks<0, 5>(mi, g, d, tmem, frame16, abort_flag, p.d_status);
         else ok = qk_chunks<5, NCH>(mi, g, d, tmem, frame16, abort_flag, p.d_status);
         if (!ok) break;
-        tc::umma_commit(&mi->s_full[WHOLE ? n % 3 : n & 1]);
+        if (tc::elect_one()) tc::umma_commit(&mi->s_full[WHOLE ? n % 3 : n & 1]);
+        __syncwarp();
         cur.next(p.segs);
       }
     }
   } else if (warp == 12) {
     // ---------------- SV issuer ----------------
-    if (lane == 0) {
+    {
       const uint64_t k_major = tc::umma_desc_sw128(0, 16, 1024);
       const uint64_t v_desc = tc::umma_desc_sw128(0, CHUNK, 1024);  // MN-major: 64-column groups one slot apart
       const uint32_t ring16 = (tc::smem_u32(s_ring) & 0x3FFFFu) >> 4;
       constexpr uint32_t id256 = tc::umma_idesc_bf16(HEADS, 256, 0, 1);
       TileCursor cur;
       cur.init(p.segs, seg0, seg1);
-      bool ok = true;
-      while (!cur.done() && ok) {
+      while (!cur.done()) {
         const int g = cur.g;
-        ok = tc::mbar_wait(&mi->p_full[cur.n % 3], (cur.n / 3) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
-        if (!ok) break;
+        if (!warp_wait(&mi->p_full[cur.n % 3], (cur.n / 3) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT)) break;
         tc::tc_fence_after();
         const uint64_t da = k_major | (uint64_t)(ring16 + (p_slot_off<NCH>(g) >> 4));
         const uint32_t acc0 = cur.t > 0 ? 1u : 0u;
+        if (tc::elect_one()) {
 #pragma unroll
-        for (int nh = 0; nh < 2; ++nh) {
-          // latent columns 256*nh .. +255 are chunks 4nh .. 4nh+3 of the tile's frame
-          const uint32_t d = tmem + LANE16 + COL_O + nh * 256;
-          const uint64_t db = v_desc | (uint64_t)(ring16 + ((g % 3) * NCH + 4 * nh) * (CHUNK / 16));
+          for (int nh = 0; nh < 2; ++nh) {
+            // latent columns 256*nh .. +255 are chunks 4nh .. 4nh+3 of the tile's frame
+            const uint32_t d = tmem + LANE16 + COL_O + nh * 256;
+            const uint64_t db = v_desc | (uint64_t)(ring16 + ((g % 3) * NCH + 4 * nh) * (CHUNK / 16));
 #pragma unroll
-          for (int k = 0; k < TILE / 16; ++k) tc::umma_bf16(d, da + k * 2, db + k * 128, id256, k > 0 ? 1u : acc0);
+            for (int k = 0; k < TILE / 16; ++k) tc::umma_bf16(d, da + k * 2, db + k * 128, id256, k > 0 ? 1u : acc0);
+          }
+          tc::umma_commit(&mi->o_done[g & 3]);
         }
-        tc::umma_commit(&mi->o_done[g & 3]);
+        __syncwarp();
         cur.next(p.segs);
       }
     }

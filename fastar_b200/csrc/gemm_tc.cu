@@ -146,21 +146,34 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
     }
   } else if (warp == 1) {
     pdl_wait();
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::umma_idesc_bf16(W_TILE, NT, W_KN ? 1 : 0, 0);
-      // descriptors differ only in the start-address field: keep the rest in registers
-      const uint64_t w_tmpl = W_KN ? tc::umma_desc_sw128(0, W_BYTES / 2, 1024) : tc::umma_desc_sw128(0, 16, 1024);
-      const uint64_t a_tmpl = tc::umma_desc_sw128(0, 16, 1024);
-      // 14-bit start-address field: inside a cluster the shared-window address of a CTA carries
-      // its rank in high bits, which must not leak into the neighbouring descriptor fields
-      const uint32_t base = tc::smem_u32(smem) & 0x3FFFFu;
-      bool ok = true;
-      for (int i = 0; i < n_kc && ok; ++i) {
-        const int s = i % p.stages;
-        ok = tc::mbar_wait(&full[s], (i / p.stages) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT);
-        if (!ok) break;
-        tc::tc_fence_after();
-        const uint32_t w16 = (base + s * STAGE_BYTES) >> 4, a16 = w16 + (W_BYTES >> 4);
+    // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow the
+    // descriptors stay in uniform registers (an MMA every 30 cycles; from a lane-0 branch every 65).
+    // The next stage's barrier is asked before this stage's MMAs are issued, so that its answer
+    // (about 200 cycles) is there when they are: 680 -> 300 cycles per stage, which with few tokens
+    // was more than the stage's bytes need.
+    constexpr uint32_t idesc = tc::umma_idesc_bf16(W_TILE, NT, W_KN ? 1 : 0, 0);
+    // descriptors differ only in the start-address field: keep the rest in registers
+    const uint64_t w_tmpl = W_KN ? tc::umma_desc_sw128(0, W_BYTES / 2, 1024) : tc::umma_desc_sw128(0, 16, 1024);
+    const uint64_t a_tmpl = tc::umma_desc_sw128(0, 16, 1024);
+    // 14-bit start-address field: inside a cluster the shared-window address of a CTA carries
+    // its rank in high bits, which must not leak into the neighbouring descriptor fields
+    const uint32_t base16 = (tc::smem_u32(smem) & 0x3FFFFu) >> 4;
+    bool ok = true;
+    int s = 0;
+    uint32_t parity = 0;
+    bool ready = n_kc > 0 && tc::mbar_try_wait(&full[0], 0);
+    for (int i = 0; i < n_kc; ++i) {
+      if (!__all_sync(0xffffffffu, ready))
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], parity, abort_flag, p.d_status, ST_MMA_TIMEOUT));
+      if (!ok) break;
+      const uint32_t w16 = base16 + s * (STAGE_BYTES >> 4), a16 = w16 + (W_BYTES >> 4);
+      uint64_t* done = &empty[s];
+      if (++s == p.stages) {
+        s = 0;
+        parity ^= 1;
+      }
+      ready = i + 1 < n_kc && tc::mbar_test_wait(&full[s], parity);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
           // K-major: 16 k = 32 bytes along the row; MN-major: 16 k rows of 128 bytes
@@ -168,9 +181,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
           const uint64_t db = a_tmpl | (uint64_t)(a16 + k * 2);
           tc::umma_bf16(tmem, da, db, idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
-        tc::umma_commit(&empty[s]);  // the stage is free once these MMAs have read it
+        tc::umma_commit(done);  // the stage is free once these MMAs have read it
+        if (i + 1 == n_kc) tc::umma_commit(acc_bar);
       }
-      if (ok) tc::umma_commit(acc_bar);
+      __syncwarp();
     }
   } else {
     // epilogue warps: TMEM lane quadrant = warp % 4; thread = one weight row n
