@@ -334,45 +334,47 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
   pdl_wait();  // Q_eff and the appended cache rows come from earlier kernels
 
   if (warp == 0 || warp == 10 || warp == 11) {
-    // ---------------- TMA producers: lane 0 of warps 0, 10, 11 ----------------
+    // ---------------- TMA producers: warps 0, 10, 11 (one elected lane each) ----------------
     // Tile g goes to ring frame g % 3, which is free once the SV MMAs of tile g-3 have retired;
     // chunk c of the tile is copied by producer (g * NCH + c) % 3.  The chunks of a tile land in three groups (one
     // chunk of each producer per group), each with its own barrier, so that the QK MMAs of the
     // first group run while the rest of the tile is still on its way.
-    if (lane == 0) {
+    {
       const int r = warp == 0 ? 0 : warp - 9;
-      if (r == 0) {
+      if (r == 0 && lane == 0) {
         tc::tma_prefetch_desc(&tmKV);
         tc::tma_prefetch_desc(&tmQ);
       }
       TileCursor cur;
       cur.init(p.segs, seg0, seg1);
-      bool ok = true;
       // cache tiles are read once and are more than L2 holds: they leave L2 first, so that the
       // partials written here are still there when the merge reads them -- unless the schedule
       // has the lanes of a group read the same tiles side by side (blocks of query tokens)
       const uint64_t stream_policy = p.tiles_shared ? tc::l2_policy_evict_normal() : tc::l2_policy_evict_first();
       // the chunks of slot g that this producer copies, from rows row0 .. row0+63 of `map`
       auto fill = [&](int g, const CUtensorMap* map, int row0) -> bool {
-        const int c0 = (r + 3 - (g * NCH) % 3) % 3;
-        if (g >= 3 && !tc::mbar_wait(&mi->o_done[(g - 3) & 3], ((g - 3) >> 2) & 1, abort_flag, p.d_status, ST_TMA_TIMEOUT))
+        if (g >= 3 && !warp_wait(&mi->o_done[(g - 3) & 3], ((g - 3) >> 2) & 1, abort_flag, p.d_status, ST_TMA_TIMEOUT))
           return false;
-        for (int c = c0; c < NCH; c += 3) {
-          const int slot = (g % 3) * NCH + c;
-          tc::mbar_expect_tx(&mi->full_t[g & 3][c / 3], CHUNK);
-          tc::tma_load_3d_hint(s_ring + slot * CHUNK, map, &mi->full_t[g & 3][c / 3], c * 64, row0, 0, stream_policy);
+        if (tc::elect_one()) {
+          const int c0 = (r + 3 - (g * NCH) % 3) % 3;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int c = c0 + 3 * i;
+            if (c < NCH) {
+              tc::mbar_expect_tx(&mi->full_t[g & 3][i], CHUNK);
+              tc::tma_load_3d_hint(s_ring + ((g % 3) * NCH + c) * CHUNK, map, &mi->full_t[g & 3][i], c * 64, row0, 0, stream_policy);
+            }
+          }
         }
+        __syncwarp();
         return true;
       };
-      while (!cur.done() && ok) {
+      while (!cur.done()) {
         // a segment opens with the Q_eff block of its token (64 rows of q_eff)
-        if (cur.t == 0) {
-          ok = fill(cur.gq, &tmQ, cur.sg.tok * HEADS);
-          if (!ok) break;
-        }
+        if (cur.t == 0 && !fill(cur.gq, &tmQ, cur.sg.tok * HEADS)) break;
         const int32_t* table = p.tables + cur.sg.table;
         const int row0 = table[(cur.sg.kv_begin >> 6) + cur.t] * TILE;
-        ok = fill(cur.g, &tmKV, row0);
+        if (!fill(cur.g, &tmKV, row0)) break;
         cur.next(p.segs);
       }
     }

@@ -108,41 +108,51 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
+    // (warp-uniform code, one elected lane issues: see the MMA issuer)
     if (lane == 0) {
       tc::tma_prefetch_desc(&tmW);
       tc::tma_prefetch_desc(&tmA);
-      auto load_w = [&](int i) {
-        const int s = i % p.stages;
-        unsigned char* st = smem + (size_t)s * STAGE_BYTES;
-        const int k0 = (kc0 + i) * BK;
-        tc::mbar_expect_tx(&full[s], STAGE_BYTES);
-        if (W_KN) {
-          // two boxes of [64 k rows x 64 n]: n is the innermost coordinate
-          tc::tma_load_3d(st, &tmW, &full[s], n0, k0, z);
-          tc::tma_load_3d(st + W_BYTES / 2, &tmW, &full[s], n0 + 64, k0, z);
-        } else {
-          tc::tma_load_3d(st, &tmW, &full[s], k0, p.w_swap ? z : n0, p.w_swap ? n0 : z);
-        }
-      };
-      auto load_a = [&](int i) {
-        const int s = i % p.stages;
-        tc::tma_load_3d(smem + (size_t)s * STAGE_BYTES + W_BYTES, &tmA, &full[s], (kc0 + i) * BK, p.a_swap ? z : m0,
-                        p.a_swap ? m0 : z);
-      };
-      // Weights are written by no kernel: the first ring of weight tiles is requested while the
-      // previous kernel still runs; the activations are its output and wait for it.
-      const int first = min(n_kc, p.stages);
-      for (int i = 0; i < first; ++i) load_w(i);
-      pdl_launch();
-      pdl_wait();
-      for (int i = 0; i < first; ++i) load_a(i);
-      for (int i = first; i < n_kc; ++i) {
-        if (!tc::mbar_wait(&empty[i % p.stages], ((i / p.stages) - 1) & 1, abort_flag, p.d_status, ST_TMA_TIMEOUT)) break;
-        load_w(i);
-        load_a(i);
+    }
+    auto load_w = [&](int i, int s) {
+      unsigned char* st = smem + (size_t)s * STAGE_BYTES;
+      const int k0 = (kc0 + i) * BK;
+      tc::mbar_expect_tx(&full[s], STAGE_BYTES);
+      if (W_KN) {
+        // two boxes of [64 k rows x 64 n]: n is the innermost coordinate
+        tc::tma_load_3d(st, &tmW, &full[s], n0, k0, z);
+        tc::tma_load_3d(st + W_BYTES / 2, &tmW, &full[s], n0 + 64, k0, z);
+      } else {
+        tc::tma_load_3d(st, &tmW, &full[s], k0, p.w_swap ? z : n0, p.w_swap ? n0 : z);
       }
-    } else {
-      pdl_wait();
+    };
+    auto load_a = [&](int i, int s) {
+      tc::tma_load_3d(smem + (size_t)s * STAGE_BYTES + W_BYTES, &tmA, &full[s], (kc0 + i) * BK, p.a_swap ? z : m0,
+                      p.a_swap ? m0 : z);
+    };
+    // Weights are written by no kernel: the first ring of weight tiles is requested while the
+    // previous kernel still runs; the activations are its output and wait for it.
+    const int first = min(n_kc, p.stages);
+    for (int i = 0; i < first; ++i)
+      if (tc::elect_one()) load_w(i, i);
+    __syncwarp();
+    pdl_launch();
+    pdl_wait();
+    for (int i = 0; i < first; ++i)
+      if (tc::elect_one()) load_a(i, i);
+    __syncwarp();
+    int s = 0;
+    uint32_t parity = 0;
+    for (int i = first; i < n_kc; ++i) {
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], parity, abort_flag, p.d_status, ST_TMA_TIMEOUT))) break;
+      if (tc::elect_one()) {
+        load_w(i, s);
+        load_a(i, s);
+      }
+      __syncwarp();
+      if (++s == p.stages) {
+        s = 0;
+        parity ^= 1;
+      }
     }
   } else if (warp == 1) {
     pdl_wait();
