@@ -48,8 +48,8 @@ constexpr uint32_t LANE16 = 16u << 16;
 constexpr float RESCALE_THRESHOLD = 8.0f;
 
 // Shared memory: a ring of three tile frames (NCH chunk slots each); with eight chunks per tile
-// three P buffers behind it (with nine, P lives in the frame's ninth chunk, see below); the
-// staging area of the epilogue; barriers and small arrays.  227 KB either way.
+// three P buffers behind it (with nine, P lives in the frame's ninth chunk, see below); barriers and
+// small arrays.  219 KB either way.
 //
 // Where P lives.  The probabilities of a tile (64 heads x 64 tokens bf16, 8 KB) are the A operand
 // of its SV MMAs.  Every tile has a P buffer of its own, with the life of its ring frame: for
@@ -60,10 +60,8 @@ constexpr float RESCALE_THRESHOLD = 8.0f;
 // buffer it had to); it waits for them only in the rare case that it rescales O.  Worth 1.3 us
 // of 85 on the batched-decode workload: the kernel is not bound by that dependency.
 constexpr int MISC_BYTES = 2048;
-constexpr int STAGE_BYTES = 8192;
 __host__ __device__ constexpr int off_pbuf(int nch) { return 3 * nch * CHUNK; }
-__host__ __device__ constexpr int off_stage(int nch) { return 3 * nch * CHUNK + (nch == 9 ? 0 : 3 * P_BYTES); }
-__host__ __device__ constexpr int off_misc(int nch) { return off_stage(nch) + STAGE_BYTES; }
+__host__ __device__ constexpr int off_misc(int nch) { return 3 * nch * CHUNK + (nch == 9 ? 0 : 3 * P_BYTES); }
 __host__ __device__ constexpr int smem_total(int nch) { return off_misc(nch) + MISC_BYTES + 1024; }
 // byte offset (from the ring base) of the P buffer of the tile in ring slot g
 template <int NCH>
@@ -160,6 +158,11 @@ __device__ __forceinline__ void tmem_ld16x32(uint32_t taddr, float* v) {
 __device__ __forceinline__ void tmem_st16x32(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.st.sync.aligned.16x32bx2.x16.b32 [%16], 16, {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
                ::"r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])), "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void st_global_v8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
+               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -307,7 +310,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_ring = smem;
-  unsigned char* s_stage = smem + off_stage(NCH);
   StreamMisc* mi = reinterpret_cast<StreamMisc*>(smem + off_misc(NCH));
   volatile int* abort_flag = &mi->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -331,6 +333,11 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
   tc::tc_fence_after();
   const uint32_t tmem = mi->tmem_slot;
   pdl_launch();
+  // The schedule and the block tables are the plan's: the first segment and the page of its first
+  // tile are looked up before the wait (two dependent round trips of 0.7-0.9 us behind it otherwise).
+  TileCursor cur;
+  cur.init(p.segs, seg0, seg1);
+  int page = cur.done() ? 0 : p.tables[cur.sg.table + (cur.sg.kv_begin >> 6)];
   pdl_wait();  // Q_eff and the appended cache rows come from earlier kernels
 
   if (warp == 0 || warp == 10 || warp == 11) {
@@ -345,8 +352,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
         tc::tma_prefetch_desc(&tmKV);
         tc::tma_prefetch_desc(&tmQ);
       }
-      TileCursor cur;
-      cur.init(p.segs, seg0, seg1);
       // cache tiles are read once and are more than L2 holds: they leave L2 first, so that the
       // partials written here are still there when the merge reads them -- unless the schedule
       // has the lanes of a group read the same tiles side by side (blocks of query tokens)
@@ -372,10 +377,9 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
       while (!cur.done()) {
         // a segment opens with the Q_eff block of its token (64 rows of q_eff)
         if (cur.t == 0 && !fill(cur.gq, &tmQ, cur.sg.tok * HEADS)) break;
-        const int32_t* table = p.tables + cur.sg.table;
-        const int row0 = table[(cur.sg.kv_begin >> 6) + cur.t] * TILE;
-        if (!fill(cur.g, &tmKV, row0)) break;
+        if (!fill(cur.g, &tmKV, page * TILE)) break;
         cur.next(p.segs);
+        if (!cur.done()) page = p.tables[cur.sg.table + (cur.sg.kv_begin >> 6) + cur.t];
       }
     }
   } else if (warp == 1 || warp == 13) {
@@ -388,8 +392,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
     {
       const int part = warp == 1 ? 0 : 1;
       const uint32_t ring16 = (tc::smem_u32(s_ring) & 0x3FFFFu) >> 4;
-      TileCursor cur;
-      cur.init(p.segs, seg0, seg1);
       bool ok = true;
       while (!cur.done() && ok) {
         const int g = cur.g, n = cur.n;
@@ -426,8 +428,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
       const uint64_t v_desc = tc::umma_desc_sw128(0, CHUNK, 1024);  // MN-major: 64-column groups one slot apart
       const uint32_t ring16 = (tc::smem_u32(s_ring) & 0x3FFFFu) >> 4;
       constexpr uint32_t id256 = tc::umma_idesc_bf16(HEADS, 256, 0, 1);
-      TileCursor cur;
-      cur.init(p.segs, seg0, seg1);
       while (!cur.done()) {
         const int g = cur.g;
         if (!warp_wait(&mi->p_full[cur.n % 3], (cur.n / 3) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT)) break;
@@ -459,9 +459,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
     const int sub = lane >> 4;
     const int row = quad * 16 + (lane & 15);
     const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
-    // epilogue staging: half of the P rows of this quadrant (what the two warps of the quadrant
-    // write during the softmax, so the quadrant barrier orders the two uses)
-    unsigned char* stage = s_stage + quad * 2048 + half * 1024;
     // The Q_eff block in ring slot gq -> tensor memory (bf16 pairs, two dims per column).  The block
     // came through the ring like a tile, ahead of the segment's first tile, so it does not queue
     // behind the tiles in flight as loads by these threads would.  Every QK MMA of the previous
@@ -504,8 +501,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
       tc::mbar_arrive(&mi->q_ready);
       return true;
     };
-    TileCursor cur;
-    cur.init(p.segs, seg0, seg1);
     bool ok = true;
     while (!cur.done() && ok) {
       const AttnSeg sg = cur.sg;
@@ -615,63 +610,20 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
           p.part_l[(long long)sg.part * HEADS + row] = mi->lsum[0][row] + mi->lsum[1][row];
           p.part_m[(long long)sg.part * HEADS + row] = m_used * 0.6931471805599453f;  // back to ln units
         }
-        {
-          // A 32-lane load hands lanes 16-31 the O rows of this quadrant (row lane-16), 32 columns
-          // at a time; this warp owns columns 256*half .. +255.  The rows go through shared memory
-          // so that every store instruction writes four full 128-byte lines.
-          float* po = p.part_o + ((long long)sg.part * HEADS + quad * 16) * D_V + half * 256;
-          if (cur.done()) {
-            // The CTA's last segment: every tile has retired, so the ring is idle and each warp
-            // stages its whole 16 x 256 block there (16 KB) -- all tensor-memory loads first, one
-            // warp barrier, then the stores back to back instead of 16 small round trips.
-            unsigned char* big = s_ring + (warp - 2) * 16384;
+        // Straight from tensor memory: a thread owns 32 consecutive columns of one head and stores them
+        // as four whole 32-byte sectors (through a shared-memory transpose, with four full lines per
+        // store instruction, the last partial of a block took 4.5 us on the kernel's critical path).
+        float* po = p.part_o + ((long long)sg.part * HEADS + row) * D_V + half * 256 + sub * 32;
 #pragma unroll 1
-            for (int cc = 0; cc < 8; ++cc) {
-              float o[32];
-              tc::tmem_ld32(lane_addr + COL_O + half * 256 + cc * 32, o);
-              if (sub == 1) {
-                const int rr = lane - 16;
+        for (int cc = 0; cc < 4; ++cc) {
+          float o[32];
+          tmem_ld16x64(lane_addr + LANE16 + COL_O + half * 256 + cc * 64, o);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                  *reinterpret_cast<float4*>(big + cc * 2048 + rr * 128 + ((u ^ (rr & 7)) * 16)) =
-                      make_float4(o[u * 4], o[u * 4 + 1], o[u * 4 + 2], o[u * 4 + 3]);
-              }
-            }
-            __syncwarp();
-#pragma unroll 4
-            for (int i = 0; i < 32; ++i) {
-              const int cc = i >> 2, rr = (i & 3) * 4 + (lane >> 3), u = lane & 7;
-              const float4 v = *reinterpret_cast<const float4*>(big + cc * 2048 + rr * 128 + ((u ^ (rr & 7)) * 16));
-              *reinterpret_cast<float4*>(po + (long long)rr * D_V + cc * 32 + u * 4) = v;
-            }
-          } else {
-#pragma unroll 1
-            for (int cc = 0; cc < 8; ++cc) {
-              float o[32];
-              tc::tmem_ld32(lane_addr + COL_O + half * 256 + cc * 32, o);
-#pragma unroll
-              for (int h8 = 0; h8 < 2; ++h8) {  // eight rows at a time through the 1 KB staging area
-                if (sub == 1 && ((lane >> 3) & 1) == h8) {
-                  const int rr = lane & 7;
-#pragma unroll
-                  for (int u = 0; u < 8; ++u)
-                    *reinterpret_cast<float4*>(stage + rr * 128 + ((u ^ rr) * 16)) = make_float4(o[u * 4], o[u * 4 + 1], o[u * 4 + 2], o[u * 4 + 3]);
-                }
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  const int rr = i * 4 + (lane >> 3), u = lane & 7;
-                  const float4 v = *reinterpret_cast<const float4*>(stage + rr * 128 + ((u ^ rr) * 16));
-                  *reinterpret_cast<float4*>(po + (long long)(h8 * 8 + rr) * D_V + cc * 32 + u * 4) = v;
-                }
-                __syncwarp();
-              }
-            }
-          }
+          for (int u = 0; u < 4; ++u) st_global_v8(po + cc * 64 + u * 8, o + u * 8);
         }
       }
       tc::tc_fence_before();
-      ok = quad_bar_and(quad, ok);  // lsum, the staging rows and O are reused by the next segment
+      ok = quad_bar_and(quad, ok);  // lsum and O are reused by the next segment
     }
   }
 
