@@ -351,8 +351,8 @@ def measure_longctx(a, torch, dist, timer, rank, world, local):
 
 
 def measure_noalloc(torch, rows=65536, calls=10):
-    """fst_cuda_mla_attention_noalloc (decode attention without a context or any allocation, CUDA-core
-    kernels, at most 31 splits: its scratch is a fixed 4 MiB array) at its largest size: us per call."""
+    """fst_cuda_mla_attention_noalloc (decode attention without a context or any allocation, its
+    partials in a fixed 18.6 MiB array) at its largest size: us per call."""
     from fastar_b200 import mla
     g = torch.Generator(device="cuda").manual_seed(0)
     cache = torch.randn((rows, 576), generator=g, device="cuda").to(torch.bfloat16)

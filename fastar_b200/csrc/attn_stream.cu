@@ -91,6 +91,7 @@ struct StreamParams {
   const float* lut;         // [T, rope] (cos, sin): inverse RoPE of the output tail of heads 0 .. inv_rope-1
   int rope, inv_rope;
   int tiles_shared;  // other blocks read the same tiles at about the same time: normal L2 priority
+  int flat_rows;     // FLAT: cached rows of the one contiguous sequence
 };
 
 
@@ -180,6 +181,9 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
 // position it tracks, so that all roles agree on (segment, tile in segment, running tile index).
 // The ring carries SLOTS: every segment puts its Q_eff block (64 heads x d_qk, the geometry of a
 // page) into one slot, followed by one slot per tile.
+// FLAT: one query token over one contiguous cache; block k's only segment is the k-th of gridDim.x
+// equal runs of pages, worked out here instead of read from a schedule in memory.
+template <bool FLAT>
 struct TileCursor {
   int si, seg_end;   // current segment, one past the CTA's last
   int t, n_tiles;    // tile within the segment, tiles of the segment
@@ -188,24 +192,40 @@ struct TileCursor {
   int n;             // running tile index (slots that are tiles)
   int sidx;          // running segment index
   AttnSeg sg;
-  __device__ __forceinline__ void load(const AttnSeg* segs) {
+  __device__ __forceinline__ void load(const StreamParams& p) {
     if (si < seg_end) {
-      sg = segs[si];
+      if (FLAT) {
+        const int tiles = (p.flat_rows + TILE - 1) / TILE;
+        sg.tok = 0;
+        sg.table = 0;
+        sg.part = si;
+        sg.kv_begin = (int)((long long)tiles * si / gridDim.x) * TILE;
+        sg.kv_end = min(p.flat_rows, (int)((long long)tiles * (si + 1) / gridDim.x) * TILE);
+      } else {
+        sg = p.segs[si];
+      }
       // kv_begin is page aligned except at the edge of a sliding window
       n_tiles = (sg.kv_end - (sg.kv_begin & ~(TILE - 1)) + TILE - 1) / TILE;
       gq = g++;
     }
   }
-  __device__ __forceinline__ void init(const AttnSeg* segs, int seg0, int seg1) {
-    si = seg0; seg_end = seg1; t = 0; g = 0; gq = 0; n = 0; sidx = 0; n_tiles = 0;
-    load(segs);
+  __device__ __forceinline__ void init(const StreamParams& p) {
+    si = FLAT ? (int)blockIdx.x : p.cta_seg[blockIdx.x];
+    seg_end = FLAT ? si + 1 : p.cta_seg[blockIdx.x + 1];
+    t = 0; g = 0; gq = 0; n = 0; sidx = 0; n_tiles = 0;
+    load(p);
+  }
+  // pool page of the current tile
+  __device__ __forceinline__ int page(const StreamParams& p) const {
+    const int i = (sg.kv_begin >> 6) + t;
+    return FLAT ? i : p.tables[sg.table + i];
   }
   __device__ __forceinline__ bool done() const { return si >= seg_end; }
-  __device__ __forceinline__ void next(const AttnSeg* segs) {
+  __device__ __forceinline__ void next(const StreamParams& p) {
     ++g; ++n;
     if (++t == n_tiles) {
       t = 0; ++si; ++sidx;
-      load(segs);
+      load(p);
     }
   }
 };
@@ -304,7 +324,7 @@ __device__ __forceinline__ bool qk_chunks(StreamMisc* mi, int g, uint32_t d, uin
 // waiting for it to free a buffer -- the better trade when tiles come from L2 (blocks of query
 // tokens: the kernel is bound by its own pipeline there; attention of the 32 x 16 x 16384 verify block
 // 1.69 -> 1.55 ms), the worse one when the life of a frame bounds the kernel (decode: 86 -> 88 us).
-template <int NCH, bool DIRECT, bool WHOLE>
+template <int NCH, bool DIRECT, bool WHOLE, bool FLAT>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmQ, StreamParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -313,7 +333,6 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
   StreamMisc* mi = reinterpret_cast<StreamMisc*>(smem + off_misc(NCH));
   volatile int* abort_flag = &mi->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int seg0 = p.cta_seg[blockIdx.x], seg1 = p.cta_seg[blockIdx.x + 1];
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 4; ++i) {
@@ -335,9 +354,9 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
   pdl_launch();
   // The schedule and the block tables are the plan's: the first segment and the page of its first
   // tile are looked up before the wait (two dependent round trips of 0.7-0.9 us behind it otherwise).
-  TileCursor cur;
-  cur.init(p.segs, seg0, seg1);
-  int page = cur.done() ? 0 : p.tables[cur.sg.table + (cur.sg.kv_begin >> 6)];
+  TileCursor<FLAT> cur;
+  cur.init(p);
+  int page = cur.done() ? 0 : cur.page(p);
   pdl_wait();  // Q_eff and the appended cache rows come from earlier kernels
 
   if (warp == 0 || warp == 10 || warp == 11) {
@@ -378,8 +397,8 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
         // a segment opens with the Q_eff block of its token (64 rows of q_eff)
         if (cur.t == 0 && !fill(cur.gq, &tmQ, cur.sg.tok * HEADS)) break;
         if (!fill(cur.g, &tmKV, page * TILE)) break;
-        cur.next(p.segs);
-        if (!cur.done()) page = p.tables[cur.sg.table + (cur.sg.kv_begin >> 6) + cur.t];
+        cur.next(p);
+        if (!cur.done()) page = cur.page(p);
       }
     }
   } else if (warp == 1 || warp == 13) {
@@ -402,7 +421,7 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
           if (ok && part == 0 && lane == 0) tc::mbar_arrive(&mi->o_done[cur.gq & 3]);
         }
         if (WHOLE && (n & 1) != part) {  // the other issuer's tile
-          cur.next(p.segs);
+          cur.next(p);
           continue;
         }
         const int k = WHOLE ? n : 2 * n + part, buf = k % 3, use = k / 3;
@@ -418,7 +437,7 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
         if (!ok) break;
         if (tc::elect_one()) tc::umma_commit(&mi->s_full[WHOLE ? n % 3 : n & 1]);
         __syncwarp();
-        cur.next(p.segs);
+        cur.next(p);
       }
     }
   } else if (warp == 12) {
@@ -446,7 +465,7 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
           tc::umma_commit(&mi->o_done[g & 3]);
         }
         __syncwarp();
-        cur.next(p.segs);
+        cur.next(p);
       }
     }
   } else {
@@ -510,7 +529,7 @@ k_attn_stream(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ 
       if (cur.sidx == 0) ok = write_q(cur.gq);
       float m_used = -INFINITY, l = 0.0f;
       int g = cur.g;
-      for (int t = 0; t < n_tiles && ok; ++t, cur.next(p.segs)) {
+      for (int t = 0; t < n_tiles && ok; ++t, cur.next(p)) {
         g = cur.g;
         const int n = cur.n;
         ok = tc::mbar_wait(&mi->s_full[WHOLE ? n % 3 : n & 1], (WHOLE ? n / 3 : n >> 1) & 1, abort_flag, p.d_status, ST_SOFTMAX_TIMEOUT);
@@ -652,7 +671,7 @@ cudaError_t launch_attn_stream(const AttnArgs& a, cudaStream_t st) {
   static_assert(sizeof(StreamMisc) <= MISC_BYTES, "misc region too small");
   static_assert(smem_total(9) <= 227 * 1024 && smem_total(8) <= 227 * 1024, "shared memory budget");
   static_assert(COL_S + 3 * TILE <= TMEM_COLS, "tensor memory budget");
-  if (a.n_segs <= 0) return cudaSuccess;
+  if (a.n_segs <= 0 && a.flat_rows <= 0) return cudaSuccess;
   CUtensorMap tmKV;
   const char* err = nullptr;
   if (!tc::cached_tmap(&tmKV, a.pool, (uint64_t)a.row, (uint64_t)a.pool_rows, 1, (uint64_t)a.row * 2,
@@ -673,15 +692,17 @@ cudaError_t launch_attn_stream(const AttnArgs& a, cudaStream_t st) {
   p.tok_part = a.tok_part; p.o_lat = a.o_lat; p.sinks = a.sinks; p.lut = a.lut;
   p.rope = a.rope; p.inv_rope = a.inv_rope;
   p.tiles_shared = a.tiles_shared ? 1 : 0;
+  p.flat_rows = a.flat_rows;
   const bool whole = a.tiles_shared;
-#define FST_ATTN_LAUNCH(NCHV, DIR, WH) \
-  launch_k(a.dependent_launch, k_attn_stream<NCHV, DIR, WH>, dim3(a.n_ctas), dim3(ST_THREADS), smem_total(NCHV), st, 1, tmKV, tmQ, p)
+#define FST_ATTN_LAUNCH(NCHV, DIR, WH, FL) \
+  launch_k(a.dependent_launch, k_attn_stream<NCHV, DIR, WH, FL>, dim3(a.n_ctas), dim3(ST_THREADS), smem_total(NCHV), st, 1, tmKV, tmQ, p)
+  if (a.flat_rows > 0) return a.d_qk == 576 ? FST_ATTN_LAUNCH(9, false, false, true) : FST_ATTN_LAUNCH(8, false, false, true);
   if (a.d_qk == 576) {
-    if (whole) return p.direct ? FST_ATTN_LAUNCH(9, true, true) : FST_ATTN_LAUNCH(9, false, true);
-    return p.direct ? FST_ATTN_LAUNCH(9, true, false) : FST_ATTN_LAUNCH(9, false, false);
+    if (whole) return p.direct ? FST_ATTN_LAUNCH(9, true, true, false) : FST_ATTN_LAUNCH(9, false, true, false);
+    return p.direct ? FST_ATTN_LAUNCH(9, true, false, false) : FST_ATTN_LAUNCH(9, false, false, false);
   }
-  if (whole) return p.direct ? FST_ATTN_LAUNCH(8, true, true) : FST_ATTN_LAUNCH(8, false, true);
-  return p.direct ? FST_ATTN_LAUNCH(8, true, false) : FST_ATTN_LAUNCH(8, false, false);
+  if (whole) return p.direct ? FST_ATTN_LAUNCH(8, true, true, false) : FST_ATTN_LAUNCH(8, false, true, false);
+  return p.direct ? FST_ATTN_LAUNCH(8, true, false, false) : FST_ATTN_LAUNCH(8, false, false, false);
 #undef FST_ATTN_LAUNCH
 }
 

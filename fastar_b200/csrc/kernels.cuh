@@ -173,10 +173,13 @@ struct AttnArgs {
   // for callers whose schedule arrays (segs, cta_seg, tables) are WRITTEN by that kernel: the
   // attention kernel reads its block's segment range before it waits for its predecessor.
   bool dependent_launch = true;
-  // the schedule makes several thread blocks read the same cache tiles at about the same time
-  // (blocks of query tokens): tiles then keep the normal L2 priority instead of leaving first, and
+  // several thread blocks read the same cache tiles while these are in L2 (a prompt, or lanes side by side in
+  // blocks of query tokens): tiles then keep the normal L2 priority instead of leaving first, and
   // the tcgen05 kernel lets each QK issuer take whole tiles (k_attn_stream, WHOLE)
   bool tiles_shared = false;
+  // tcgen05 kernel only, 0 = off: one query token over one contiguous cache of this many rows, cut
+  // into n_ctas equal runs of pages, block k writing partial k; no schedule arrays are read.
+  int flat_rows = 0;
   // tcgen05 kernel only: a token whose whole context is ONE segment of the schedule (one partial)
   // is normalised and written to o_lat by the attention kernel itself and leaves no partial; the
   // merge kernel that follows is told to skip such tokens (MergeArgs::skip_single).
@@ -205,7 +208,8 @@ struct MergeArgs {
   int T, H, d_v, rope, inv_rope, mode;
   int threads;              // 128: rows have few parts (a thread per 4 columns); otherwise 256 (8 warps share the parts)
   int skip_single = 0;      // rows of tokens with exactly one partial are already in o_lat (AttnArgs::direct_single)
-  int wide = 0;             // few rows with many parts each: a block per (row, 128 columns) instead of per row
+  int flat_parts = 0;       // > 0: one token with this many partials from slot 0 on (tok_part is not read)
+  int wide = 0;             // many parts per row: a block per (row, 128 columns) instead of per row
 };
 void launch_merge(const MergeArgs& a, cudaStream_t st);
 

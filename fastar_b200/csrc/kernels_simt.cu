@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(256) k_merge_wide(MergeArgs a) {
   __shared__ float s_red[16];
   const int r = blockIdx.x, cg = blockIdx.y, t = r / a.H, h = r % a.H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p0 = a.tok_part[t], n_parts = a.tok_part[t + 1] - p0;
+  const int p0 = a.flat_parts ? 0 : a.tok_part[t], n_parts = a.flat_parts ? a.flat_parts : a.tok_part[t + 1] - p0;
   if (a.skip_single && n_parts == 1) return;
   const bool sk = a.sinks != nullptr;
   float M = sk ? a.sinks[h] : -INFINITY;

@@ -23,23 +23,24 @@ constexpr int NA_MAX_ROWS = 65536;   // cached rows
 constexpr int NA_MAX_HEADS = 64;
 constexpr int NA_MAX_DV = 512;
 constexpr int NA_MAX_DQK = 576;
-constexpr int NA_MAX_SPLITS = 32;    // KV splits = thread blocks of the attention kernel
+constexpr int NA_MAX_SPLITS = 148;   // KV splits = thread blocks of the attention kernel: one per SM
 constexpr int NA_PAGE = 64;
+constexpr int NA_PAGES_PER_BLOCK = 2;
 
 // Layout of the scratch array (byte offsets, all multiples of 256).
 constexpr size_t OFF_PART_O = 0;
-constexpr size_t SZ_PART_O = (size_t)NA_MAX_SPLITS * NA_MAX_HEADS * NA_MAX_DV * sizeof(float);  // 4 MiB
+constexpr size_t SZ_PART_O = (size_t)NA_MAX_SPLITS * NA_MAX_HEADS * NA_MAX_DV * sizeof(float);  // 18.5 MiB
 constexpr size_t OFF_PART_M = OFF_PART_O + SZ_PART_O;
 constexpr size_t SZ_PART_ML = (size_t)NA_MAX_SPLITS * NA_MAX_HEADS * sizeof(float);
 constexpr size_t OFF_PART_L = OFF_PART_M + SZ_PART_ML;
 constexpr size_t OFF_SEGS = OFF_PART_L + SZ_PART_ML;
-constexpr size_t OFF_TABLE = OFF_SEGS + 1024;                                   // 32 segments x 20 bytes, padded
-constexpr size_t OFF_TOK = OFF_TABLE + (NA_MAX_ROWS / NA_PAGE) * sizeof(int32_t);  // tok_table[1], tok_part[2]; from
-                                                                                // int 16: cta_seg[33]; int 60: status
+constexpr size_t OFF_TABLE = OFF_SEGS + 3072;                                   // 148 segments x 20 bytes, padded
+constexpr size_t OFF_TOK = OFF_TABLE + (NA_MAX_ROWS / NA_PAGE) * sizeof(int32_t);  // tok_table[1], tok_part[2];
+                                                                                // int 60: status
 constexpr size_t OFF_LUT = OFF_TOK + 256;                                       // unused RoPE table slot
 constexpr size_t SCRATCH_BYTES = OFF_LUT + 256;
 
-// Every GPU that loads the library holds this array (about 4.02 MiB) until the process exits.
+// Every GPU that loads the library holds this array (about 18.6 MiB) until the process exits.
 static __device__ __align__(256) unsigned char g_na_scratch[SCRATCH_BYTES];
 
 // Device address of g_na_scratch per device.  In host code the array's name is only a
@@ -47,10 +48,10 @@ static __device__ __align__(256) unsigned char g_na_scratch[SCRATCH_BYTES];
 // cudaGetSymbolAddress, asked once per device with that device current.
 unsigned char* g_na_ptr[64] = {nullptr};
 
-// Rewrites every piece of bookkeeping the attention and merge kernels read from the scratch:
-// an identity block table (the cache is contiguous), the split schedule, the one-token maps.
-// unit: rows per schedule tile -- 32 for the CUDA-core kernel, 64 (a page) for the tcgen05 one,
-// whose thread block k walks segment k (cta_seg) and reports a wait that ran out in the status word.
+// Rewrites every piece of bookkeeping the CUDA-core attention kernel and its merge read from the
+// scratch: an identity block table (the cache is contiguous), the split schedule, the one-token
+// maps.  (The tcgen05 kernel works its run out from the block index: AttnArgs::flat_rows.)
+// unit: rows per schedule tile.
 __global__ void k_na_setup(unsigned char* scratch, int n_rows, int n_splits, int unit) {
   AttnSeg* segs = reinterpret_cast<AttnSeg*>(scratch + OFF_SEGS);
   int32_t* table = reinterpret_cast<int32_t*>(scratch + OFF_TABLE);
@@ -69,12 +70,10 @@ __global__ void k_na_setup(unsigned char* scratch, int n_rows, int n_splits, int
     sg.table = 0;  // the identity block table starts at entry 0
     segs[s] = sg;
   }
-  if (threadIdx.x <= n_splits) tok[16 + threadIdx.x] = threadIdx.x;  // cta_seg: block k takes segment k
   if (threadIdx.x == 0) {
     tok[0] = 0;         // tok_table[0]: the token's block table starts at entry 0
     tok[1] = 0;         // tok_part[0]
     tok[2] = n_splits;  // tok_part[1]
-    tok[60] = 0;        // status word of the bounded waits
   }
 }
 
@@ -128,7 +127,7 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   a.pool = static_cast<const bf16*>(d_cache);
   a.tables = reinterpret_cast<const int32_t*>(sc + OFF_TABLE);
   a.segs = reinterpret_cast<const AttnSeg*>(sc + OFF_SEGS);
-  a.cta_seg = reinterpret_cast<const int32_t*>(sc + OFF_TOK) + 16;
+  a.cta_seg = nullptr;
   a.part_m = reinterpret_cast<float*>(sc + OFF_PART_M);
   a.part_l = reinterpret_cast<float*>(sc + OFF_PART_L);
   a.part_o = reinterpret_cast<float*>(sc + OFF_PART_O);
@@ -142,21 +141,24 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   a.pool_rows = n_rows;
   a.scale = softmax_scale;
   // The full MLA shape (64 heads, 576- or 512-wide rows, 512 value columns) goes to the tcgen05
-  // streaming kernel, one thread block per split over whole 64-row pages; every other shape to the
-  // CUDA-core kernel (so do caches of less than one page).  Either way at most 32 splits: that is
-  // what the scratch holds.
+  // streaming kernel, one thread block per run of whole 64-row pages; every other shape to the
+  // CUDA-core kernel (so do caches of less than one page) on at most 32 blocks.
+  // A block streams about 40 bytes per clock, so the pages are spread over every SM -- but no thinner
+  // than NA_PAGES_PER_BLOCK pages each: every block leaves 128 KB of partials behind.  With 32 blocks
+  // and the schedule written by a kernel in front 20 000 rows took 32.8 us, now 26.0.
   const bool stream = n_rows >= NA_PAGE && attn_stream_supported(a);
-  const int unit = stream ? NA_PAGE : 32;
-  const int n_splits = std::max(1, std::min(NA_MAX_SPLITS, stream ? (n_rows + NA_PAGE - 1) / NA_PAGE : (n_rows + 127) / 128));
+  const int n_pages = (n_rows + NA_PAGE - 1) / NA_PAGE;
+  const int n_splits = stream ? std::max(1, std::min(NA_MAX_SPLITS, (n_pages + NA_PAGES_PER_BLOCK - 1) / NA_PAGES_PER_BLOCK))
+                              : std::max(1, std::min(32, (n_rows + 127) / 128));
   a.n_segs = n_splits;
   a.n_ctas = n_splits;
-  k_na_setup<<<1, 256, 0, st>>>(sc, n_rows, n_splits, unit);
   if (stream) {
-    // (not as a programmatic dependent: the schedule it reads on entry was written by k_na_setup)
+    a.flat_rows = n_rows;
     a.dependent_launch = false;
     cudaError_t es = launch_attn_stream(a, st);
     if (es != cudaSuccess) return na_fail(FST_MLA_ERR_CUDA, cudaGetErrorString(es));
   } else {
+    k_na_setup<<<1, 256, 0, st>>>(sc, n_rows, n_splits, 32);
     launch_attn_simt(a, st);
   }
 
@@ -176,6 +178,7 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   m.inv_rope = 0;
   m.mode = 0;
   m.threads = 256;
+  m.flat_parts = stream ? n_splits : 0;
   m.wide = 1;  // one query token: a block per (head row, 128 columns) where the shape allows
   launch_merge(m, st);
   cudaError_t e = cudaGetLastError();

@@ -378,7 +378,7 @@ int fst_cuda_mla_debug_attr_first_use(uint64_t kernel_key, int32_t device, int64
  * = softmax(scale * q K^T) V, no sink.  Both inputs 16-byte aligned.  Work is enqueued on
  * cuda_stream (NULL: default stream) of the current device; the call does not synchronise.
  *
- * The split-KV partials live in a fixed array inside the library image (about 4 MiB, held by
+ * The split-KV partials live in a fixed array inside the library image (about 18.6 MiB, held by
  * every GPU that loads the library until the process exits), hence the limits: n_rows <= 65536,
  * n_heads <= 64, d_qk <= 576 (multiple of 8), d_v <= 512 (multiple of 64, <= d_qk).  Anything
  * larger returns FST_MLA_ERR_CAPACITY (fst_cuda_mla_last_error says why); use the context API
