@@ -34,6 +34,7 @@ struct GemmTcParams {
   int M, N, K, ldc;
   long long c_bs;
   int splits, kc_total, stages;
+  int nt, n_tiles, m_tiles, tiles;  // k_gemm_tc_tiles: token tile, weight / token tiles, tiles of all batch members
   int w_swap, a_swap;  // the batch index is the middle tensor-map coordinate (its stride is the smaller one)
   // side job (GemmArgs::rope_*): null source = none
   const bf16* rope_src;
@@ -87,6 +88,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
   const int n0 = blockIdx.x * W_TILE;
   const int m_tile = blockIdx.y / p.splits, split = blockIdx.y % p.splits;
   const int m0 = m_tile * NT;
+  // tokens that the MMAs and the reduction cover: with the largest tile, no padding beyond 16
+  const int n_cols = NT == 256 ? min(NT, (p.M - m0 + 15) & ~15) : NT;
   const int z = blockIdx.z;
   const int kc0 = (int)((long long)p.kc_total * split / p.splits);
   const int kc1 = (int)((long long)p.kc_total * (split + 1) / p.splits);
@@ -161,7 +164,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
     // The next stage's barrier is asked before this stage's MMAs are issued, so that its answer
     // (about 200 cycles) is there when they are: 680 -> 300 cycles per stage, which with few tokens
     // was more than the stage's bytes need.
-    constexpr uint32_t idesc = tc::umma_idesc_bf16(W_TILE, NT, W_KN ? 1 : 0, 0);
+    uint32_t idesc = tc::umma_idesc_bf16(W_TILE, NT, W_KN ? 1 : 0, 0);
+    if (NT == 256) idesc = tc::umma_idesc_bf16(W_TILE, 16, W_KN ? 1 : 0, 0) + ((uint32_t)((n_cols - 16) >> 3) << 17);
     // descriptors differ only in the start-address field: keep the rest in registers
     const uint64_t w_tmpl = W_KN ? tc::umma_desc_sw128(0, W_BYTES / 2, 1024) : tc::umma_desc_sw128(0, 16, 1024);
     const uint64_t a_tmpl = tc::umma_desc_sw128(0, 16, 1024);
@@ -289,7 +293,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
     } else if (ok) {
       float* red = reinterpret_cast<float*>(smem);  // [NT][128]: the ring is idle once acc_bar fired
       for (int c0 = 0; c0 < NT; c0 += 32) {
-        if (p.splits == 1 && m0 + c0 >= p.M) break;
+        if (p.splits == 1 ? m0 + c0 >= p.M : c0 >= n_cols) break;
         float v[32];
         if (n_kc > 0) {
           tc::tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + c0, v);
@@ -319,7 +323,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
     // cluster, peers in rank order
     cluster_sync_all();
     const uint32_t rank = cluster_ctarank();
-    const int c_lo = (int)(NT * rank / p.splits), c_hi = (int)(NT * (rank + 1) / p.splits);
+    const int c_lo = (int)(n_cols * rank / p.splits), c_hi = (int)(n_cols * (rank + 1) / p.splits);
     const uint32_t red_addr = tc::smem_u32(smem);
     for (int e4 = c_lo * (W_TILE / 4) + threadIdx.x; e4 < c_hi * (W_TILE / 4); e4 += GEMM_THREADS) {
       const int col = e4 / (W_TILE / 4), row = (e4 % (W_TILE / 4)) * 4;
@@ -368,6 +372,308 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUten
   }
 }
 
+// Many tokens: a persistent kernel, one block (or pair of blocks) per SM (or pair).  A block walks output
+// tiles (128 weight rows x up to 256 tokens, no K split); the accumulator is double-buffered in tensor
+// memory and two groups of four epilogue warps take alternate tiles, so the operand ring and the tensor
+// pipe run on while earlier tiles leave.  With a block per tile every tile paid its own start-up, first
+// round trip and drain, 12-15 us a wave whatever its K.
+//
+// PAIR: two SMs share a tile of 256 weight rows (tcgen05 cta_group::2).  Each block fetches its own 128
+// weight rows and HALF of the tokens, the MMAs read both halves, and each block's tensor memory gets its
+// own rows of the product: 32 KB instead of 48 KB per block and K chunk.  What an SM can fetch, 55 bytes
+// a clock, bounds the single-block form (891 cycles per chunk of 512 MMA cycles at K = 8192).  The leader
+// (rank 0) issues; both blocks' copies report to the leader's barriers, its commits to the barriers of both.
+constexpr int PG_THREADS = 320;          // warps: 0 copies, 1 issues MMAs, 2-5 and 6-9 the two epilogue groups
+constexpr int PG_NT = 256;               // largest token tile
+constexpr int PG_RING = 192 * 1024;      // operand ring
+constexpr int PG_MAX_STAGES = 7;
+constexpr int PG_OUT = 32 * W_TILE * 2;  // 32 tokens x 128 weight rows of bf16
+constexpr int PG_SMEM = PG_RING + 4 * PG_OUT + 1024 /* alignment */ + 256 /* barriers */;
+
+__device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(tc::smem_u32(p)), "r"(rank));
+  return remote;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// One arrival at the barrier of this offset in both blocks of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(tc::smem_u32(bar)), "h"((uint16_t)3)
+               : "memory");
+}
+
+template <bool W_KN, bool PAIR>
+__global__ void __launch_bounds__(PG_THREADS, 1)
+k_gemm_tc_tiles(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, GemmTcParams p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* s_out = smem + PG_RING;  // [group][2][32 tokens][128]
+  uint64_t* full = reinterpret_cast<uint64_t*>(s_out + 4 * PG_OUT);
+  uint64_t* empty = full + PG_MAX_STAGES;
+  uint64_t* acc_full = empty + PG_MAX_STAGES;
+  uint64_t* acc_empty = acc_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int COLS = PAIR ? 2 * W_TILE : W_TILE;  // weight rows per tile
+  const int rank = PAIR ? (int)cluster_ctarank() : 0;
+  const int worker = PAIR ? blockIdx.x >> 1 : blockIdx.x, n_workers = PAIR ? gridDim.x >> 1 : gridDim.x;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      tc::mbar_init(&acc_full[a], 1);
+      tc::mbar_init(&acc_empty[a], PAIR ? 8 : 4);  // one arrival per epilogue warp
+    }
+    *abort_flag = 0;
+    tc::fence_barrier_init();
+  }
+  if (warp == 1) {
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(2 * PG_NT) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tc::tmem_alloc(tmem_slot, 2 * PG_NT);
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();  // the peer's barriers exist
+  tc::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int n_kc = p.kc_total, stage_bytes = W_BYTES + p.nt * BK * 2 / (PAIR ? 2 : 1);
+  // tokens that the MMAs of a tile cover: a ragged last tile multiplies no padding
+  auto tile_cols = [&](int m0) { return PAIR ? min(p.nt, (p.M - m0 + 31) & ~31) : min(p.nt, (p.M - m0 + 15) & ~15); };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tc::tma_prefetch_desc(&tmW);
+      tc::tma_prefetch_desc(&tmA);
+    }
+    const uint32_t full0 = PAIR ? mapa_u32(&full[0], 0) : 0;
+    auto load = [&](void* dst, const CUtensorMap* map, int s, int x, int y, int z) {
+      if (PAIR) tma_load_3d_pair(dst, map, full0 + s * 8, x, y, z);
+      else tc::tma_load_3d(dst, map, &full[s], x, y, z);
+    };
+    auto load_w = [&](int tile, int kc, int s) {
+      unsigned char* st = smem + s * stage_bytes;
+      const int n0 = (tile % p.n_tiles) * COLS + rank * W_TILE, z = tile / p.n_tiles / p.m_tiles, k0 = kc * BK;
+      if (rank == 0) tc::mbar_expect_tx(&full[s], PAIR ? 2 * stage_bytes : stage_bytes);
+      if (W_KN) {
+        load(st, &tmW, s, n0, k0, z);
+        load(st + W_BYTES / 2, &tmW, s, n0 + 64, k0, z);
+      } else {
+        load(st, &tmW, s, k0, p.w_swap ? z : n0, p.w_swap ? n0 : z);
+      }
+    };
+    auto load_a = [&](int tile, int kc, int s) {
+      int m0 = tile / p.n_tiles % p.m_tiles * p.nt;
+      const int z = tile / p.n_tiles / p.m_tiles;
+      if (PAIR && rank) m0 += tile_cols(m0) / 2;
+      load(smem + s * stage_bytes + W_BYTES, &tmA, s, kc * BK, p.a_swap ? z : m0, p.a_swap ? m0 : z);
+    };
+    // the first weight tiles before the wait for the kernel ahead (no kernel writes weights)
+    const int first = min(n_kc, p.stages);
+    for (int i = 0; i < first; ++i)
+      if (tc::elect_one()) load_w(worker, i, i);
+    __syncwarp();
+    pdl_launch();
+    pdl_wait();
+    for (int i = 0; i < first; ++i)
+      if (tc::elect_one()) load_a(worker, i, i);
+    __syncwarp();
+    int s = first % p.stages;
+    uint32_t parity = first == p.stages ? 0 : 1;  // of the stage's last use; the first ring has none
+    bool ok = true;
+    for (int tile = worker, kc = first; tile < p.tiles && ok; tile += n_workers, kc = 0) {
+      for (; kc < n_kc; ++kc) {
+        // (parity 1 on a fresh barrier: passes at once)
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[s], parity, abort_flag, p.d_status, ST_TMA_TIMEOUT));
+        if (!ok) break;
+        if (tc::elect_one()) {
+          load_w(tile, kc, s);
+          load_a(tile, kc, s);
+        }
+        __syncwarp();
+        if (++s == p.stages) {
+          s = 0;
+          parity ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1 && rank == 0) {
+    // (warp-uniform walk, one elected lane issues, the next stage's barrier asked ahead: as in k_gemm_tc)
+    const uint64_t w_tmpl = W_KN ? tc::umma_desc_sw128(0, W_BYTES / 2, 1024) : tc::umma_desc_sw128(0, 16, 1024);
+    const uint64_t a_tmpl = tc::umma_desc_sw128(0, 16, 1024);
+    const uint32_t base16 = (tc::smem_u32(smem) & 0x3FFFFu) >> 4;
+    int s = 0, i = 0;
+    uint32_t parity = 0;
+    bool ok = true, ready = tc::mbar_try_wait(&full[0], 0);
+    for (int tile = worker; tile < p.tiles && ok; tile += n_workers, ++i) {
+      const int m0 = tile / p.n_tiles % p.m_tiles * p.nt;
+      const uint32_t idesc = tc::umma_idesc_bf16(COLS, 16, W_KN ? 1 : 0, 0) + ((uint32_t)((tile_cols(m0) - 16) >> 3) << 17);
+      const uint32_t d = tmem + (i & 1) * PG_NT;
+      if (i >= 2) {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_empty[i & 1], ((i >> 1) - 1) & 1, abort_flag, p.d_status, ST_MMA_TIMEOUT));
+        if (!ok) break;
+      }
+      tc::tc_fence_after();
+      for (int kc = 0; kc < n_kc; ++kc) {
+        if (!__all_sync(0xffffffffu, ready))
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], parity, abort_flag, p.d_status, ST_MMA_TIMEOUT));
+        if (!ok) break;
+        const uint32_t w16 = base16 + s * (stage_bytes >> 4), a16 = w16 + (W_BYTES >> 4);
+        uint64_t* done = &empty[s];
+        if (++s == p.stages) {
+          s = 0;
+          parity ^= 1;
+        }
+        ready = tc::mbar_test_wait(&full[s], parity);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t dw = w_tmpl | (uint64_t)(w16 + (W_KN ? k * 128 : k * 2));
+            const uint64_t da = a_tmpl | (uint64_t)(a16 + k * 2);
+            if (PAIR) umma_bf16_pair(d, dw, da, idesc, (kc > 0 || k > 0) ? 1u : 0u);
+            else tc::umma_bf16(d, dw, da, idesc, (kc > 0 || k > 0) ? 1u : 0u);
+          }
+          if (PAIR) umma_commit_pair(done);
+          else tc::umma_commit(done);
+          if (kc + 1 == n_kc) {
+            if (PAIR) umma_commit_pair(&acc_full[i & 1]);
+            else tc::umma_commit(&acc_full[i & 1]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp >= 2) {
+    pdl_wait();
+    const uint32_t acc_empty0 = PAIR ? mapa_u32(&acc_empty[0], 0) : 0;
+    const int group = (warp - 2) >> 2, quad = warp & 3, et = (threadIdx.x - 64) & 127;
+    if (p.rope_src) {
+      // RoPE of the query's rope dims, four pairs (16 bytes) per item, spread over all blocks (32-bit index
+      // arithmetic: the divisions are most of an item's instructions)
+      const uint32_t per_row = p.rope_dims / 8;
+      const uint32_t n_items = p.rope_T * p.rope_H * per_row, step = gridDim.x * 256;
+      for (uint32_t i0 = blockIdx.x * 256 + (threadIdx.x - 64); i0 < n_items; i0 += 4 * step) {
+        uint4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t i = i0 + u * step, row = i / per_row;
+          if (i < n_items)
+            x[u] = *reinterpret_cast<const uint4*>(p.rope_src + (long long)row * p.rope_q_head + p.rope_nope + (i - row * per_row) * 8);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t i = i0 + u * step, row = i / per_row;
+          if (i < n_items) {
+            const uint32_t v = i - row * per_row;
+            const float* lut = p.rope_lut + (long long)(row / (uint32_t)p.rope_H) * p.rope_dims + v * 8;
+            uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
+              const float x0 = __low2float(b), x1 = __high2float(b), c = lut[2 * e], sn = lut[2 * e + 1];
+              const __nv_bfloat162 r = __floats2bfloat162_rn(x0 * c - x1 * sn, x0 * sn + x1 * c);
+              w[e] = *reinterpret_cast<const uint32_t*>(&r);
+            }
+            *reinterpret_cast<uint4*>(p.rope_dst + (long long)row * p.rope_d_qk + p.rope_d_qk - p.rope_dims + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+    }
+    unsigned char* out = s_out + group * 2 * PG_OUT;
+    const int row = quad * 32 + lane;
+    int buf = 0;
+    for (int tile = worker + group * n_workers, use = 0; tile < p.tiles; tile += 2 * n_workers, ++use) {
+      const int n0 = (tile % p.n_tiles) * COLS + rank * W_TILE, m0 = tile / p.n_tiles % p.m_tiles * p.nt, z = tile / p.n_tiles / p.m_tiles;
+      const bool ok = tc::mbar_wait(&acc_full[group], use & 1, abort_flag, p.d_status, ST_EPI_TIMEOUT);
+      // the four warps of a group go on together or not at all
+      uint32_t all_ok;
+      asm volatile(
+          "{\n\t.reg .pred q, r;\n\t"
+          "setp.ne.u32 q, %1, 0;\n\t"
+          "bar.red.and.pred r, %2, 128, q;\n\t"
+          "selp.u32 %0, 1, 0, r;\n\t}"
+          : "=r"(all_ok)
+          : "r"((uint32_t)ok), "r"(1 + group)
+          : "memory");
+      if (!all_ok) break;
+      tc::tc_fence_after();
+      const int n_tok = min(p.nt, p.M - m0);
+      bf16* c = p.C + z * p.c_bs + (long long)m0 * p.ldc + n0;
+      for (int c0 = 0; c0 < n_tok; c0 += 32) {
+        float v[32];
+        tc::tmem_ld32(tmem + group * PG_NT + ((uint32_t)(quad * 32) << 16) + c0, v);
+        if (c0 + 32 >= n_tok) {  // the accumulator has been read
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (PAIR) mbar_arrive_cluster(acc_empty0 + group * 8);
+            else tc::mbar_arrive(&acc_empty[group]);
+          }
+        }
+        bf16* so = reinterpret_cast<bf16*>(out + buf * PG_OUT) + row;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) so[j * W_TILE] = f2bf(v[j]);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        // 16 threads per token row of 256 bytes; the next slice is staged in the other buffer, and this one
+        // is written again only behind the next barrier
+        const int r8 = (et & 15) * 8;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int tok = (et >> 4) + 8 * q;
+          if (c0 + tok < n_tok && n0 + r8 < p.N)
+            *reinterpret_cast<uint4*>(c + (long long)(c0 + tok) * p.ldc + r8) =
+                *reinterpret_cast<const uint4*>(out + buf * PG_OUT + tok * (W_TILE * 2) + r8 * 2);
+        }
+        buf ^= 1;
+      }
+    }
+  }
+
+  __syncwarp();
+  tc::tc_fence_before();
+  __syncthreads();
+  if (p.status_host && threadIdx.x == 0) {
+    const int st = *reinterpret_cast<const volatile int*>(p.status_dev);
+    if (st != 0) *reinterpret_cast<volatile int*>(p.status_host) = st;
+  }
+  if (*abort_flag) {
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // let copies and MMAs in flight settle
+  }
+  if (PAIR) {
+    __syncwarp();
+    cluster_sync_all();  // nobody leaves while the peer may still signal its barriers
+  }
+  if (warp == 1) {
+    tc::tc_fence_after();
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PG_NT) : "memory");
+    else tc::tmem_dealloc(tmem, 2 * PG_NT);
+  }
+}
+
 int pick_nt(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256; }
 
 template <int NT, bool W_KN>
@@ -395,20 +701,46 @@ cudaError_t launch_gemm_tc(const GemmArgs& g, int* d_status, cudaStream_t st) {
   n_sm = sm_count[dev & 63];
   int NT = pick_nt(g.M);
   const int n_tiles = (g.N + W_TILE - 1) / W_TILE;
-  // a 256-token tile leaves no room for the parked partial: use it only when no K split is needed
-  if (NT == 256 && (long long)n_tiles * ((g.M + 255) / 256) * g.batch * 2 <= 2ll * n_sm) NT = 128;
   const int m_tiles = (g.M + NT - 1) / NT;
   const int kc_total = (g.K + BK - 1) / BK;
   // K slices (a power of two, one cluster) while two CTAs per SM are not yet covered, keeping
   // at least two K chunks per CTA
   const long long tiles = (long long)n_tiles * m_tiles * g.batch;
   int splits = 1;
-  while (splits < MAX_SPLITS && tiles * splits * 2 <= 2ll * n_sm && kc_total / (splits * 2) >= 2) splits *= 2;
+  // -- or, with more than 128 tokens, while there is one per SM: a block then streams its K slice of 128
+  // weight rows and of all its tokens (up to 256).  Two tiles of 128 tokens fetched every weight row twice:
+  // 192 tokens, 4096 x 4096 27.1 -> 24.6 us; 512 tokens, 4096 x 8192 45.8 -> 40.2.
+  const long long room = NT == 256 ? n_sm : 2ll * n_sm;
+  while (splits < MAX_SPLITS && tiles * splits * 2 <= room && kc_total / (splits * 2) >= 2) splits *= 2;
   // Output tiles that cover half of the SMs or more are not split at all: a block per SM with a ring
   // of eight stages and no cluster reduction beats two half-size blocks on a third of the SMs
   // (the q-expand GEMM, 96 tiles: 18.2 -> 16.5 us; cut in three or four it was slower still).
   // With a handful of tokens the split wins (one token: 14.5 against 16.3 us).
-  if (NT >= 64 && tiles * 2 >= n_sm && tiles <= n_sm) splits = 1;
+  if (NT >= 64 && NT < 256 && tiles * 2 >= n_sm && tiles <= n_sm) splits = 1;
+
+  // Enough tokens and output tiles to give every SM one without a K split: the persistent kernel, with
+  // the token tile (a multiple of 32) whose rounds of tiles fetch least: a tile's operands are its 128
+  // weight rows and its tokens.  It stores 16 bytes at a time and rotates 16 bytes at a time.
+  const bool persistent = g.M > 128 && splits == 1 && g.N % 8 == 0 && g.ldc % 8 == 0 && g.c_bs % 8 == 0 &&
+                          (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
+                          (!g.rope_src || (g.rope_q_head % 8 == 0 && g.rope_nope % 8 == 0 && g.rope_dims % 8 == 0 && g.rope_d_qk % 8 == 0 &&
+                                           (long long)g.rope_T * g.rope_H * g.rope_dims < (1ll << 31) &&
+                                           (reinterpret_cast<uintptr_t>(g.rope_src) & 15) == 0 && (reinterpret_cast<uintptr_t>(g.rope_dst) & 15) == 0));
+  // Pairs of blocks fetch less per MMA; a product of one weight tile (the value projection of a head)
+  // would leave the second block of every pair idle, and an odd tile number half of the last one.
+  const bool pair = persistent && (n_tiles % 2 == 0 || n_tiles >= 8);
+  const int cols = pair ? (n_tiles + 1) / 2 : n_tiles, workers = pair ? n_sm / 2 : n_sm;
+  if (persistent) {
+    long long best = 0;
+    for (int nt = PG_NT; nt >= 128; nt -= 32) {
+      const long long rounds = ((long long)cols * ((g.M + nt - 1) / nt) * g.batch + workers - 1) / workers;
+      const int fetch = W_TILE + (pair ? nt / 2 : nt);
+      if (best == 0 || rounds * fetch < best) {
+        best = rounds * fetch;
+        NT = nt;
+      }
+    }
+  }
 
   CUtensorMap tmW, tmA;
   const char* err = nullptr;
@@ -432,7 +764,7 @@ cudaError_t launch_gemm_tc(const GemmArgs& g, int* d_status, cudaStream_t st) {
   } else {
     ok = build(&tmW, g.B, g.N, g.ldb, g.b_bs, W_TILE, &w_swap);
   }
-  if (!ok || !build(&tmA, g.A, g.M, g.lda, g.a_bs, NT, &a_swap)) return cudaErrorInvalidValue;
+  if (!ok || !build(&tmA, g.A, g.M, g.lda, g.a_bs, pair ? NT / 2 : NT, &a_swap)) return cudaErrorInvalidValue;
 
   GemmTcParams p;
   p.C = g.C; p.d_status = d_status;
@@ -442,6 +774,17 @@ cudaError_t launch_gemm_tc(const GemmArgs& g, int* d_status, cudaStream_t st) {
   p.rope_T = g.rope_T; p.rope_H = g.rope_H; p.rope_q_head = g.rope_q_head; p.rope_nope = g.rope_nope;
   p.rope_dims = g.rope_dims; p.rope_d_qk = g.rope_d_qk;
   p.status_dev = g.status_host ? g.status_dev : nullptr; p.status_host = g.status_dev ? g.status_host : nullptr;
+  if (persistent) {
+    p.nt = NT; p.n_tiles = cols; p.m_tiles = (g.M + NT - 1) / NT;
+    p.tiles = cols * p.m_tiles * g.batch;
+    p.stages = std::min(PG_MAX_STAGES, PG_RING / (W_BYTES + NT * BK * 2 / (pair ? 2 : 1)));
+    const dim3 grid(std::min(p.tiles, workers) * (pair ? 2 : 1)), block(PG_THREADS);
+    if (pair)
+      return g.b_kn ? launch_pdl(k_gemm_tc_tiles<true, true>, grid, block, PG_SMEM, st, 2, tmW, tmA, p)
+                    : launch_pdl(k_gemm_tc_tiles<false, true>, grid, block, PG_SMEM, st, 2, tmW, tmA, p);
+    return g.b_kn ? launch_pdl(k_gemm_tc_tiles<true, false>, grid, block, PG_SMEM, st, 1, tmW, tmA, p)
+                  : launch_pdl(k_gemm_tc_tiles<false, false>, grid, block, PG_SMEM, st, 1, tmW, tmA, p);
+  }
   const int stage_bytes = W_BYTES + NT * BK * 2;
   // Two blocks share an SM (96 KB of operand ring each) -- unless the grid has no more blocks than
   // there are SMs: then a block has the SM to itself anyway and takes a ring that holds its whole K

@@ -52,10 +52,11 @@ inline void prefer_max_shared(const void* kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
-// Launch with programmatic stream serialisation (and an optional cluster along y).
+// Launch with programmatic stream serialisation (and an optional cluster of
+// `cluster` blocks: along y, in a one-row grid along x -- a pair for cta_group::2 has to lie along x).
 template <class... KArgs, class... Args>
 inline cudaError_t launch_k(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                            int cluster_y, Args&&... args) {
+                            int cluster, Args&&... args) {
   prefer_max_shared(reinterpret_cast<const void*>(kernel));
   cudaError_t e_attr = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e_attr != cudaSuccess) return e_attr;
@@ -71,10 +72,10 @@ inline cudaError_t launch_k(bool dependent, void (*kernel)(KArgs...), dim3 grid,
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;
   }
-  if (cluster_y > 1) {
+  if (cluster > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = 1;
-    attr[n].val.clusterDim.y = cluster_y;
+    attr[n].val.clusterDim.x = grid.y == 1 ? cluster : 1;
+    attr[n].val.clusterDim.y = grid.y == 1 ? 1 : cluster;
     attr[n].val.clusterDim.z = 1;
     ++n;
   }
@@ -86,8 +87,8 @@ inline cudaError_t launch_k(bool dependent, void (*kernel)(KArgs...), dim3 grid,
 // and orders itself behind it with griddepcontrol.wait.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              int cluster_y, Args&&... args) {
-  return launch_k(true, kernel, grid, block, smem, st, cluster_y, static_cast<Args&&>(args)...);
+                              int cluster, Args&&... args) {
+  return launch_k(true, kernel, grid, block, smem, st, cluster, static_cast<Args&&>(args)...);
 }
 
 // Strided-batched C[z][m, n] = sum_k A[z][m, k] * B[z][n, k]  (b_kn: B[z][k, n]).

@@ -99,3 +99,22 @@ def test_same_inputs_give_identical_bits(ctx):
     a = ctx.gemm(A, B)
     b = ctx.gemm(A, B)
     assert np.array_equal(a, b)
+
+
+# more than 128 tokens.  The persistent form: one token over a tile, a ragged last token tile, ragged weight
+# rows and K, several tiles per block (both accumulators reused), the [K, N] operand, a K shorter than the
+# operand ring, an odd number of weight tiles for pairs of blocks, and few enough of them for single blocks.
+# Then few tiles, split along K with the 256-token tile: one and several token tiles, a last one of one
+# token, eight, four and two slices
+@pytest.mark.parametrize("M,N,K,b_kn", [(129, 19000, 72, False), (300, 10240, 192, False), (300, 10248, 64, True),
+                                        (1111, 4104, 136, True), (1111, 8192, 584, False), (2049, 9600, 128, False),
+                                        (6001, 640, 136, False), (6001, 384, 72, True),
+                                        (192, 1600, 4096, False), (257, 2048, 1024, True), (1000, 520, 264, False)])
+def test_many_tokens(ctx, M, N, K, b_kn):
+    rng = np.random.default_rng(M + N + K)
+    # small integers: the sums are exact in fp32 (K * 9 < 2^24), only the bf16 store rounds
+    A = rng.integers(-3, 4, size=(M, K)).astype(np.float32)
+    B = rng.integers(-3, 4, size=(K, N) if b_kn else (N, K)).astype(np.float32)
+    got = ctx.gemm(synth.to_bf16_bits(A), synth.to_bf16_bits(B), b_kn=b_kn)
+    want = synth.to_bf16_bits(A @ (B if b_kn else B.T))
+    assert np.array_equal(got, want)
