@@ -6,6 +6,17 @@
 
 namespace fst {
 
+__device__ __forceinline__ uint4 pack8(const float* f) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
@@ -141,8 +152,52 @@ __global__ void __launch_bounds__(256) k_rmsnorm_rows(const bf16* x, const bf16*
   }
 }
 
+// The same, 16 bytes per load and store (two each at 4096 elements; the weights before the wait): with
+// 2-byte accesses the kernel was bound by issuing them (1111 rows of 4096: 15 -> 7 us; 5 rows 4.6 -> 3.5).
+__global__ void __launch_bounds__(256) k_rmsnorm_rows_vec(const bf16* x, const bf16* w, bf16* y, int dim, float eps) {
+  pdl_launch();
+  __shared__ float scratch[32];
+  const int tid = threadIdx.x, n_u = dim / 8;
+  const uint4* in = reinterpret_cast<const uint4*>(x + (long long)blockIdx.x * dim);
+  uint4* out = reinterpret_cast<uint4*>(y + (long long)blockIdx.x * dim);
+  uint4 g[4], v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < n_u) g[i] = reinterpret_cast<const uint4*>(w)[tid + i * 256];
+  pdl_wait();
+  float ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < n_u) v[i] = in[tid + i * 256];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < n_u) {
+      float f[8];
+      unpack8(v[i], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+    }
+  ss = block_sum(ss, scratch);
+  const float r = 1.0f / sqrtf(ss / (float)dim + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < n_u) {
+      float f[8], gw[8];
+      unpack8(v[i], f);
+      unpack8(g[i], gw);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = f[e] * r * gw[e];
+      out[tid + i * 256] = pack8(f);
+    }
+}
+
 void launch_rmsnorm_rows(const bf16* x, const bf16* w, bf16* y, int T, int dim, float eps, cudaStream_t st) {
   if (T <= 0) return;
+  // (the caller's device rows may sit at any 2-byte address: those take the scalar form)
+  if (dim % 8 == 0 && dim <= 8192 && aligned16(x) && aligned16(w) && aligned16(y)) {
+    launch_pdl(k_rmsnorm_rows_vec, dim3(T), dim3(256), 0, st, 1, x, w, y, dim, eps);
+    return;
+  }
   launch_pdl(k_rmsnorm_rows, dim3(T), dim3(256), 0, st, 1, x, w, y, dim, eps);
 }
 
@@ -226,8 +281,79 @@ __global__ void __launch_bounds__(256) k_norm_append(NormAppendArgs a) {
   }
 }
 
+// The same with 16 bytes (eight elements) per thread: the first warps take the query row, the others
+// the key row.  RoPE pairs never leave their thread, so one block barrier (the sums of squares) is
+// left of three; weights, RoPE row and destination are the plan's or the layer's and are read before
+// the wait.  One row 5.8 -> 3.7 us, 2048 rows 15.7 -> 7.8 us (each alone).
+__global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
+  pdl_launch();
+  __shared__ float scratch[32];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int q_warps = (a.q_lora / 8 + 31) / 32;  // the rest of the block has the key row
+  const bool is_q = wid < q_warps;
+  const int u = is_q ? threadIdx.x : threadIdx.x - q_warps * 32;
+  const int j0 = u * 8, dim = is_q ? a.q_lora : a.kv_lora;  // normed elements
+  const bool on = j0 < (is_q ? a.q_lora : a.row);
+  const bf16* w = is_q ? a.q_norm : a.kv_norm;
+  const bool normed = on && w && j0 < dim, rot = on && !is_q && j0 >= a.row - a.rope;
+  uint4 wv = make_uint4(0, 0, 0, 0), xv = make_uint4(0, 0, 0, 0);
+  float4 l0 = make_float4(0.f, 0.f, 0.f, 0.f), l1 = l0;
+  if (normed) wv = *reinterpret_cast<const uint4*>(w + j0);
+  if (rot) {
+    const float4* lut = reinterpret_cast<const float4*>(a.lut + (long long)t * a.rope + (j0 - (a.row - a.rope)));
+    l0 = lut[0];
+    l1 = lut[1];
+  }
+  const long long dst = a.dst_row[t];
+  pdl_wait();
+  const bf16* in = a.cmp + (long long)t * (a.q_lora + a.row) + (is_q ? 0 : a.q_lora);
+  if (on) xv = *reinterpret_cast<const uint4*>(in + j0);
+  float x[8];
+  unpack8(xv, x);
+  float ss = 0.0f;
+  if (j0 < dim) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
+  }
+  ss = warp_sum(ss);
+  if (lane == 0) scratch[wid] = ss;
+  __syncthreads();
+  ss = warp_sum((is_q ? lane < q_warps : lane >= q_warps && lane < nw) ? scratch[lane] : 0.0f);
+  const float r = 1.0f / sqrtf(ss / (float)dim + a.eps);
+  if (!on) return;
+  if (normed) {
+    float g[8];
+    unpack8(wv, g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = rbf(x[e] * r * g[e]);
+  }
+  if (rot) {
+    const float cs[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const float x0 = x[e], x1 = x[e + 1];
+      x[e] = x0 * cs[e] - x1 * cs[e + 1];
+      x[e + 1] = x0 * cs[e + 1] + x1 * cs[e];
+    }
+  }
+  const uint4 o = pack8(x);
+  if (is_q) {
+    *reinterpret_cast<uint4*>(a.qc + (long long)t * a.q_lora + j0) = o;
+  } else {
+    *reinterpret_cast<uint4*>(a.kv_new + (long long)t * a.row + j0) = o;
+    if (dst >= 0) *reinterpret_cast<uint4*>(a.pool + dst + j0) = o;
+  }
+}
+
 void launch_norm_append(const NormAppendArgs& a, cudaStream_t st) {
   if (a.T <= 0) return;
+  // (a cache row starts at a multiple of `row` elements)
+  const int threads = ((a.q_lora / 8 + 31) / 32 + (a.row / 8 + 31) / 32) * 32;
+  if (a.q_lora % 8 == 0 && a.row % 8 == 0 && a.kv_lora % 8 == 0 && a.rope % 8 == 0 && threads <= 512 && aligned16(a.cmp) &&
+      aligned16(a.q_norm) && aligned16(a.kv_norm) && aligned16(a.lut) && aligned16(a.qc) && aligned16(a.kv_new) && aligned16(a.pool)) {
+    launch_pdl(k_norm_append_vec, dim3(a.T), dim3(threads), 0, st, 1, a);
+    return;
+  }
   launch_pdl(k_norm_append, dim3(a.T), dim3(256), a.row * sizeof(float), st, 1, a);
 }
 
@@ -293,73 +419,77 @@ __global__ void __launch_bounds__(256) k_q_rope_token(QPrepArgs a) {
   }
 }
 
-// V4: a warp per (token, head) row, eight rows per block: the row (q_head <= 1024 values) stays in
-// registers, 16 bytes per lane and pass; one shuffle reduction instead of two block barriers and a
-// shared-memory round trip per row.  Same order of operations per element as k_q_prep.
+// V4: a warp takes R (token, head) rows; a row (q_head <= 256 * U values) stays in registers, 16 bytes
+// per lane and pass; one shuffle reduction instead of two block barriers and a shared-memory round
+// trip per row.  Same order of operations per element as k_q_prep.  All rows of a warp are loaded
+// before the first is reduced: with one row per warp too few bytes were in flight and the blocks too
+// short-lived (1111 tokens x 64 heads x 512: 41 -> 31 us, alone).
+template <int U, int R>
 __global__ void __launch_bounds__(256) k_q_prep_v4_rows(QPrepArgs a) {
   pdl_launch();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long r = (long long)blockIdx.x * 8 + warp;
-  if (r >= (long long)a.T * a.H) return;
-  const int t = (int)(r / a.H), h = (int)(r % a.H);
-  const uint4* in = reinterpret_cast<const uint4*>(a.q_full + r * a.q_head);
-  uint4* out = reinterpret_cast<uint4*>(a.q_eff + r * a.d_qk);
-  const float* lut = a.lut + (long long)t * a.rope;
+  const long long r0 = ((long long)blockIdx.x * 8 + warp) * R, n_rows = (long long)a.T * a.H;
   const int n_u = a.q_head / 8;
-  float x[4][8];
-  float ss = 0.0f;
+  uint4 v[R][U];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int u = lane + 32 * i;
-    if (u < n_u) {
-      const uint4 v = in[u];
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (int q = 0; q < R; ++q)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
-        x[i][2 * e] = __low2float(b);
-        x[i][2 * e + 1] = __high2float(b);
-        ss += x[i][2 * e] * x[i][2 * e] + x[i][2 * e + 1] * x[i][2 * e + 1];
+    for (int i = 0; i < U; ++i)
+      if (r0 + q < n_rows && lane + 32 * i < n_u)
+        v[q][i] = reinterpret_cast<const uint4*>(a.q_full + (r0 + q) * a.q_head)[lane + 32 * i];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const long long r = r0 + q;
+    if (r >= n_rows) return;
+    const int t = (int)(r / a.H), h = (int)(r % a.H);
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (lane + 32 * i < n_u) {
+        float x[8];
+        unpack8(v[q][i], x);
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) ss += x[e] * x[e] + x[e + 1] * x[e + 1];
       }
-    }
-  }
-  ss = warp_sum(ss);
-  const float sc = a.head_norm ? 1.0f / sqrtf(ss / (float)a.q_head + a.eps) : 1.0f;
-  const bool rot = h < a.rope_heads;
+    ss = warp_sum(ss);
+    const float sc = a.head_norm ? 1.0f / sqrtf(ss / (float)a.q_head + a.eps) : 1.0f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int u = lane + 32 * i;
-    if (u < n_u) {
-      float y[8];
+    for (int i = 0; i < U; ++i) {
+      const int u = lane + 32 * i;
+      if (u < n_u) {
+        float y[8];
+        unpack8(v[q][i], y);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = rbf(x[i][e] * sc);
-      const int j0 = 8 * u - a.nope;  // first rope dim of this unit, if not negative
-      if (rot && j0 >= 0) {
+        for (int e = 0; e < 8; ++e) y[e] = rbf(y[e] * sc);
+        const int j0 = 8 * u - a.nope;  // first rope dim of this unit, if not negative
+        if (h < a.rope_heads && j0 >= 0) {
+          const float4* lut = reinterpret_cast<const float4*>(a.lut + (long long)t * a.rope + j0);
+          const float4 l0 = lut[0], l1 = lut[1];
+          const float cs[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const float c = lut[j0 + e], sn = lut[j0 + e + 1], x0 = y[e], x1 = y[e + 1];
-          y[e] = x0 * c - x1 * sn;
-          y[e + 1] = x0 * sn + x1 * c;
+          for (int e = 0; e < 8; e += 2) {
+            const float x0 = y[e], x1 = y[e + 1];
+            y[e] = x0 * cs[e] - x1 * cs[e + 1];
+            y[e + 1] = x0 * cs[e + 1] + x1 * cs[e];
+          }
         }
+        reinterpret_cast<uint4*>(a.q_eff + r * a.d_qk)[u] = pack8(y);
       }
-      uint32_t pk[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat162 b = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
-        pk[e] = *reinterpret_cast<const uint32_t*>(&b);
-      }
-      out[u] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
   }
 }
 
 void launch_q_prep(const QPrepArgs& a, cudaStream_t st) {
   if (a.T <= 0) return;
-  if (a.v4 && a.q_head % 8 == 0 && a.q_head <= 1024 && a.nope % 8 == 0 && a.d_qk % 8 == 0 && a.rope % 2 == 0 &&
-      a.nope + a.rope == a.q_head && (reinterpret_cast<uintptr_t>(a.q_full) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(a.q_eff) & 15) == 0) {
-    launch_pdl(k_q_prep_v4_rows, dim3((unsigned)(((long long)a.T * a.H + 7) / 8)), dim3(256), 0, st, 1, a);
+  if (a.v4 && a.q_head % 8 == 0 && a.q_head <= 1024 && a.nope % 8 == 0 && a.d_qk % 8 == 0 && a.rope % 8 == 0 &&
+      a.nope + a.rope == a.q_head && aligned16(a.q_full) && aligned16(a.q_eff) && aligned16(a.lut)) {
+    // two rows per warp once that still gives every SM several blocks; short rows only (registers)
+    const long long rows = (long long)a.T * a.H;
+    if (a.q_head <= 512 && rows >= 8192)
+      launch_pdl(k_q_prep_v4_rows<2, 2>, dim3((unsigned)((rows + 15) / 16)), dim3(256), 0, st, 1, a);
+    else
+      launch_pdl(k_q_prep_v4_rows<4, 1>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, 1, a);
     return;
   }
   // (pair accesses need even offsets: q_head, nope, d_qk and rope are even in both presets)
