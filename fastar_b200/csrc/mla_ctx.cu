@@ -86,6 +86,7 @@ struct Sched {
   long long kv_rows = 0;
   int max_tok_parts = 0, min_tok_parts = 0, n_single_part = 0;
   bool by_blocks = false;  // cut_block_schedule made it: the lanes of a group read the same pages side by side
+  bool tiles_in_l2 = false;  // most reads of a cache tile are answered by L2
   // what the compressor kernel of this class reads (classes 1, 2)
   CompressTok* d_ctoks = nullptr;
   CompressStep* d_csteps = nullptr;
@@ -424,7 +425,7 @@ AttnArgs attn_args(FstMlaCtx* c, int lid, const bf16* q_eff, bool may_fuse = fal
   a.pool_rows = (long long)c->cfg.n_pages * c->cfg.page_tokens;
   a.q_rows = (long long)c->T * c->d.H;
   a.scale = c->cfg.softmax_scale;
-  a.tiles_shared = S.by_blocks;
+  a.tiles_shared = S.tiles_in_l2;
   if (may_fuse && c->fused_merge && S.n_single_part > 0) {
     a.direct_single = true;
     a.tok_part = S.d_tok_part;
@@ -1521,6 +1522,13 @@ int plan_schedule_part(FstMlaCtx* c, bool on_copy_stream) {
       S.min_tok_parts = std::min(S.min_tok_parts, np);
       S.n_single_part += np == 1;
     }
+    // Tiles come from L2 when the lanes of a group read them side by side, and when all rows that the
+    // call attends to stay resident (at most half of L2) and are read several times over, as a prompt
+    // does (2048 tokens: attention 427 -> 389 us, alone).
+    long long rows_once = 0;
+    for (const FstMlaSeqStep& step : c->pl_steps)
+      if (step.q_len > 0) rows_once += step.append ? step.pos0 + step.q_len : step.pos0;
+    S.tiles_in_l2 = S.by_blocks || (kv_rows >= 4 * rows_once && rows_once * c->d.row * (long long)sizeof(bf16) <= (64ll << 20));
     S.n_segs = S.n_parts = (int)segs.size();
     S.n_ctas = (int)cta_seg.size() - 1;
     S.kv_rows = kv_rows;
