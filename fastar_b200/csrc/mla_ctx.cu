@@ -96,6 +96,7 @@ struct Sched {
 
 constexpr int ATTN_TILE = 128;      // split boundaries are multiples of this many cached rows
 constexpr int MAX_EVENT_SETS = 256;
+constexpr int SMALL_OUT = 64;       // new rows up to which the last GEMM writes a pageable caller's output to page-locked memory
 
 struct EventSet {
   cudaEvent_t ev[FST_MLA_K_COUNT + 1];
@@ -135,6 +136,8 @@ struct FstMlaCtx {
   bf16* d_cproj = nullptr;       // [T, 2 * width] compressor projections of a call
   uint16_t* h_pinned = nullptr;  // [max_tokens, hidden] staging for the host-buffer entry point
   int* d_status = nullptr;
+  uint16_t* h_out = nullptr;  // [SMALL_OUT, hidden] page-locked output rows of small calls with a pageable h_out
+  bf16* h_out_dev = nullptr;  // the device's address of it
   const bf16* out_src = nullptr;  // where the last layer call left its output rows
   bool out_zero_copy = true;
   int* h_status = nullptr;  // page-locked copy of the status word, fetched on the stream before a sync
@@ -725,6 +728,9 @@ int fst_cuda_mla_create(const FstMlaConfig* cfg, FstMlaCtx** out) {
     cudaGetLastError();
     x->h_status_dev = nullptr;  // no mapping: the status word is copied behind every call instead
   }
+  if (!rc && (cudaHostAlloc((void**)&x->h_out, std::min<size_t>(T, SMALL_OUT) * d.hidden * sizeof(uint16_t), cudaHostAllocMapped) != cudaSuccess ||
+              cudaHostGetDevicePointer((void**)&x->h_out_dev, x->h_out, 0) != cudaSuccess))
+    rc = fail(FST_MLA_ERR_CUDA, "cudaHostAlloc failed");
   if (!rc && cudaHostAlloc((void**)&x->h_pinned, T * d.hidden * sizeof(uint16_t), cudaHostAllocDefault) != cudaSuccess)
     rc = fail(FST_MLA_ERR_CUDA, "cudaHostAlloc failed");
   if (rc) {
@@ -761,6 +767,7 @@ void fst_cuda_mla_destroy(FstMlaCtx* c) {
   if (c->fwd_ev) cudaEventDestroy(c->fwd_ev);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
+  if (c->h_out) cudaFreeHost(c->h_out);
   for (auto& es : c->ev_pool)
     for (auto& e : es.ev) cudaEventDestroy(e);
   delete c;
@@ -1694,7 +1701,11 @@ int fst_cuda_mla_forward(FstMlaCtx* c, int lid, const uint16_t* h_in, uint16_t* 
   const size_t bytes = (size_t)c->T * c->d.hidden * sizeof(uint16_t);
   // A page-locked output buffer that the device can address is written by the last GEMM itself
   // (512 KB of posted writes spread over the kernel) instead of by a copy behind it.
-  const bool zero_copy = out_direct && out_mapped && c->out_zero_copy && !c->profiling;
+  // So is a page-locked buffer of the context's own for small calls with a pageable one: the copy behind
+  // the kernels, its start and wait included, cost microseconds per call.
+  const bool small_out = !out_direct && c->T <= SMALL_OUT;
+  if (small_out) out_mapped = c->h_out_dev;
+  const bool zero_copy = (out_direct || small_out) && out_mapped && c->out_zero_copy && !c->profiling;
   c->out_src = zero_copy ? (const bf16*)out_mapped : c->d_out;
   void* out_dev = zero_copy ? out_mapped : (void*)c->d_out;
   if (two_parts) {
@@ -1717,7 +1728,7 @@ int fst_cuda_mla_forward(FstMlaCtx* c, int lid, const uint16_t* h_in, uint16_t* 
         for (int k = 0; k < 2; ++k)
           if (!c->lut_tag[k].empty()) lut_row_cached(c, k, pos0[b] + q_lens[b] + i);
   if ((rc = fst_cuda_mla_sync(c))) return rc;
-  if (!out_direct) memcpy(h_out, c->h_pinned, bytes);
+  if (!out_direct) memcpy(h_out, zero_copy ? c->h_out : c->h_pinned, bytes);
   return FST_MLA_OK;
 }
 
@@ -1827,7 +1838,7 @@ int fst_cuda_mla_get_stage(FstMlaCtx* c, int stage, uint16_t* host_out, size_t b
     case FST_MLA_STAGE_QEFF: src = c->d_qeff; n = (size_t)c->T * d.H * d.d_qk; break;
     case FST_MLA_STAGE_OLAT: src = c->d_olat; n = (size_t)c->T * d.H * d.d_v; break;
     case FST_MLA_STAGE_LOW: src = c->d_low; n = (size_t)c->T * d.low; break;
-    case FST_MLA_STAGE_OUT: src = c->out_src ? c->out_src : c->d_out; n = (size_t)c->T * d.hidden; break;
+    case FST_MLA_STAGE_OUT: src = c->out_src && !(c->out_src == c->h_out_dev && c->T > SMALL_OUT) ? c->out_src : c->d_out; n = (size_t)c->T * d.hidden; break;
     default: return fail(FST_MLA_ERR_ARG, "unknown stage %d", stage);
   }
   if (bytes != n * 2) return fail(FST_MLA_ERR_ARG, "stage %d holds %zu bytes, caller asked for %zu", stage, n * 2, bytes);
