@@ -598,11 +598,13 @@ int run_merge_local(FstMlaCtx* c, int lid, int mode, float* rank_partial, bool s
   m.sinks = (d.v4 && mode == 0) ? c->layers[lid].sinks : nullptr;
   m.lut = lut_of(c, lid); m.o_lat = c->d_olat; m.rank_partial = rank_partial;
   m.T = c->T; m.H = d.H; m.d_v = d.d_v; m.rope = d.rope; m.inv_rope = inv_rope_heads(c, lid); m.mode = mode;
-  // Up to six parts per token on average: a warp per row.  More parts than that only come with few
-  // tokens (a block or two per SM make partials): four blocks per row share the partials of a row
-  // (5 tokens x 27 parts, V4, two layers: 217 -> 214 us a step against a block per row).
+  // Up to six parts per token on average: a warp per row.  Twelve and more (a dozen tokens at most, as a
+  // block or two per SM make partials): four blocks per row share the parts of a row (5 tokens x 27 parts,
+  // V4, two layers: 217 -> 214 us a step against a block per row).  Between the two a block per row: with
+  // 24 tokens x 7 parts four of them per row cost the same step 408 -> 426 us.
   m.threads = S.n_parts <= 6 * c->T ? 128 : 256;
-  m.wide = 1;
+  // (And where rows are too few to fill the SMs with a block each.)
+  m.wide = S.n_parts >= 12 * c->T || (long long)c->T * d.H < 2ll * c->n_sm ? 1 : 0;
   launch_merge(m, c->stream);
   c->launches += 1;
   return FST_MLA_OK;
