@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
 void launch_norm_append(const NormAppendArgs& a, cudaStream_t st) {
   if (a.T <= 0) return;
   // One row keeps the scalar form: with the other one the layer call over one sequence of 131 072 rows took
-  // 102.0 instead of 99.3 us (over 4096 rows the same 135), although the kernel alone is shorter.
+  // 102.0 instead of 101.0 us (over 4096 rows the same 135), although the kernel alone is shorter.
   // (a cache row starts at a multiple of `row` elements)
   const int threads = ((a.q_lora / 8 + 31) / 32 + (a.row / 8 + 31) / 32) * 32;
   if (a.T > 1 && a.q_lora % 8 == 0 && a.row % 8 == 0 && a.kv_lora % 8 == 0 && a.rope % 8 == 0 && threads <= 512 && aligned16(a.cmp) &&
