@@ -25,6 +25,7 @@ constexpr int NA_MAX_DV = 512;
 constexpr int NA_MAX_DQK = 576;
 constexpr int NA_MAX_SPLITS = 148;   // KV splits = thread blocks of the attention kernel: one per SM
 constexpr int NA_PAGE = 64;
+constexpr int NA_MIN_SPLITS = 32;    // blocks that a cache is spread over before one takes a second page
 constexpr int NA_PAGES_PER_BLOCK = 2;
 
 // Layout of the scratch array (byte offsets, all multiples of 256).
@@ -143,12 +144,17 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   // The full MLA shape (64 heads, 576- or 512-wide rows, 512 value columns) goes to the tcgen05
   // streaming kernel, one thread block per run of whole 64-row pages; every other shape to the
   // CUDA-core kernel (so do caches of less than one page) on at most 32 blocks.
-  // A block streams about 40 bytes per clock, so the pages are spread over every SM -- but no thinner
-  // than NA_PAGES_PER_BLOCK pages each: every block leaves 128 KB of partials behind.  With 32 blocks
-  // and the schedule written by a kernel in front 20 000 rows took 32.8 us, now 26.0.
+  // A block streams about 40 bytes per clock, so the pages are spread over every SM -- but from 64 pages
+  // on no thinner than NA_PAGES_PER_BLOCK pages each: every block leaves 128 KB of partials behind.  With
+  // 32 blocks and the schedule written by a kernel in front 20 000 rows took 32.8 us, now 26.0.
+  // Up to there NA_MIN_SPLITS blocks, a page each up to 32 pages: the largest weight of a block's first
+  // page is exactly 1, that of a later page is rounded to bf16 like the others.  Two pages per block
+  // raise the error against 64 bits by a tenth (700 rows: 1.79e-3 -> 1.98e-3 of the result) and gain
+  // nothing (2000 rows: 14.35 us with 32 blocks, 14.95 with 16).
   const bool stream = n_rows >= NA_PAGE && attn_stream_supported(a);
   const int n_pages = (n_rows + NA_PAGE - 1) / NA_PAGE;
-  const int n_splits = stream ? std::max(1, std::min(NA_MAX_SPLITS, (n_pages + NA_PAGES_PER_BLOCK - 1) / NA_PAGES_PER_BLOCK))
+  const int n_splits = stream ? std::max(std::min(NA_MIN_SPLITS, n_pages),
+                                         std::min(NA_MAX_SPLITS, (n_pages + NA_PAGES_PER_BLOCK - 1) / NA_PAGES_PER_BLOCK))
                               : std::max(1, std::min(32, (n_rows + 127) / 128));
   a.n_segs = n_splits;
   a.n_ctas = n_splits;

@@ -77,6 +77,33 @@ def test_small_and_odd_shapes_against_the_cpu_oracle(heads, d_qk, d_v, n_rows):
     check_close(d_out.cpu().numpy().view(np.uint16), want, f"H={heads} d_qk={d_qk} d_v={d_v} rows={n_rows}", ulps=2)
 
 
+@pytest.mark.parametrize("d_qk", [576, 512])
+@pytest.mark.parametrize("n_rows", [128, 700, 2048])
+def test_a_page_of_its_own_keeps_its_largest_weight_exact(n_rows, d_qk):
+    """Up to 32 pages every thread block has one page, whose largest softmax weight is exactly 1.  All rows
+    are zero (score 0, value 0) but one in the second page with weight exp(score) = 200.5: walked behind the
+    first page by the same block, that weight would be rounded to bf16 (spacing 1 there) and the whole
+    output with it, by 1 / 401.  What is left here is the rounding of the 512 outputs, 2^-9 / sqrt(3) each
+    (relative): weighted over the row 5e-5, six times that is the bound."""
+    rng = np.random.default_rng(n_rows + d_qk)
+    rows = np.zeros((n_rows, d_qk), np.float32)
+    rows[100] = rng.standard_normal(d_qk)
+    bits = synth.to_bf16_bits(rows)
+    k = synth.from_bf16_bits(bits)[100].astype(np.float64)
+    q_bits = synth.to_bf16_bits(np.tile(k.astype(np.float32), (64, 1)))
+    scale = math.log(200.5) / float(k @ k)
+    d_rows, d_q = torch.from_numpy(bits.view(np.int16)).cuda(), torch.from_numpy(q_bits.view(np.int16)).cuda()
+    d_out = torch.zeros((64, 512), dtype=torch.int16, device="cuda")
+    rc = mla.attention_noalloc(d_q.data_ptr(), d_rows.data_ptr(), n_rows, 64, d_qk, 512, scale, d_out.data_ptr(),
+                               torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    got = synth.from_bf16_bits(d_out.cpu().numpy().view(np.uint16)).astype(np.float64)
+    want = k[:512] * 200.5 / (200.5 + n_rows - 1)
+    err = np.abs(got @ want / (want @ want) - 1)
+    assert err.max() <= 3e-4, err.max()
+
+
 def test_refusals_reach_the_last_error_string():
     d = torch.zeros(64 * 576, dtype=torch.int16, device="cuda")
     p = d.data_ptr()
