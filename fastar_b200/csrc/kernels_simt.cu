@@ -283,10 +283,14 @@ __global__ void __launch_bounds__(256) k_norm_append(NormAppendArgs a) {
 
 // The same with 16 bytes (eight elements) per thread: the first warps take the query row, the others
 // the key row.  RoPE pairs never leave their thread, so one block barrier (the sums of squares) is
-// left of three; weights, RoPE row and destination are the plan's or the layer's and are read before
-// the wait.  One row 5.8 -> 3.7 us, 2048 rows 15.7 -> 7.8 us (each alone).
+// left of three.  One row 5.8 -> 3.7 us, 2048 rows 15.7 -> 7.8 us (each alone).  Nothing is loaded before
+// the wait, although weights, RoPE row and destination could be.  Layer calls with these loads beside the
+// GEMM in front, against the scalar kernel and against this one: BASELINE, one row over 131 072 rows 105.2
+// (scalar 102.5) on one box, 100.3 (this one 100.1; scalar 101.1) on others; V4, five tokens, two layers
+// 209.0 (210.3).  What one form loses there is more than the other gains.
 __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
   pdl_launch();
+  pdl_wait();
   __shared__ float scratch[32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int q_warps = (a.q_lora / 8 + 31) / 32;  // the rest of the block has the key row
@@ -305,7 +309,6 @@ __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
     l1 = lut[1];
   }
   const long long dst = a.dst_row[t];
-  pdl_wait();
   const bf16* in = a.cmp + (long long)t * (a.q_lora + a.row) + (is_q ? 0 : a.q_lora);
   if (on) xv = *reinterpret_cast<const uint4*>(in + j0);
   float x[8];
@@ -347,11 +350,11 @@ __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
 
 void launch_norm_append(const NormAppendArgs& a, cudaStream_t st) {
   if (a.T <= 0) return;
-  // One row keeps the scalar form: with the other one the layer call over one sequence of 131 072 rows took
-  // 102.0 instead of 101.0 us (over 4096 rows the same 135), although the kernel alone is shorter.
-  // (a cache row starts at a multiple of `row` elements)
+  // The scalar form is for sizes and addresses that 16-byte accesses cannot take, never for a number of
+  // rows: the two add the squares in different orders, and a row must not depend on what else is in
+  // its call.  (A cache row starts at a multiple of `row` elements.)
   const int threads = ((a.q_lora / 8 + 31) / 32 + (a.row / 8 + 31) / 32) * 32;
-  if (a.T > 1 && a.q_lora % 8 == 0 && a.row % 8 == 0 && a.kv_lora % 8 == 0 && a.rope % 8 == 0 && threads <= 512 && aligned16(a.cmp) &&
+  if (a.q_lora % 8 == 0 && a.row % 8 == 0 && a.kv_lora % 8 == 0 && a.rope % 8 == 0 && threads <= 512 && aligned16(a.cmp) &&
       aligned16(a.q_norm) && aligned16(a.kv_norm) && aligned16(a.lut) && aligned16(a.qc) && aligned16(a.kv_new) && aligned16(a.pool)) {
     launch_pdl(k_norm_append_vec, dim3(a.T), dim3(threads), 0, st, 1, a);
     return;

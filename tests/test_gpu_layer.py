@@ -180,6 +180,30 @@ def test_yarn_rope_tables(impl, preset, by_call):
     run_layer(preset, impl, [60, 4090], 8, True, seed=6, ulps=2, rope_yarn=True, yarn_by_layer_call=by_call)
 
 
+@pytest.mark.parametrize("preset", [mla.PRESET_BASELINE, mla.PRESET_FASTAR_V4], ids=["baseline", "v4"])
+def test_a_row_does_not_depend_on_the_other_rows_of_its_call(preset):
+    """Compression, norms and key rotation of 320 tokens, 16 to a call and one to a call: the same bits (up to
+    16 tokens share the GEMM's token tile and K split, and every row goes through the same norm kernel)."""
+    n = 16
+    cfg = mla.make_config(preset, n_pages=n + 2, max_tokens=n, max_seqs=n)
+    bits, _ = weights_for(preset)
+    with mla.MlaContext(cfg) as ctx:
+        ctx.set_layer_weights(0, bits)
+        seqs = [ctx.seq_alloc() for _ in range(n)]
+        for rep in range(20):
+            h = synth.to_bf16_bits(synth.hidden_f32(cfg, 100 + rep, n))
+            ctx.append_rows(0, h, seqs, [0] * n, [1] * n)
+            qc = ctx.get_stage(mla.STAGE_QC).reshape(n, -1).copy()
+            kv = ctx.get_stage(mla.STAGE_KV).reshape(n, -1).copy()
+            for t, s in enumerate(seqs):
+                ctx.seq_truncate(s, 0)
+                ctx.append_rows(0, h[t:t + 1], [s], [0], [1])
+                assert np.array_equal(ctx.get_stage(mla.STAGE_QC).reshape(-1), qc[t]), (rep, t)
+                assert np.array_equal(ctx.get_stage(mla.STAGE_KV).reshape(-1), kv[t]), (rep, t)
+            for s in seqs:
+                ctx.seq_truncate(s, 0)
+
+
 def test_yarn_and_plain_tables_differ_on_the_device():
     """A context with one plain and one YaRN layer keeps both tables per plan; the same weights and
     rows give different q_eff / kv in the rope dims only."""
