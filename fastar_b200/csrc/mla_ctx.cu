@@ -96,7 +96,12 @@ struct Sched {
 
 constexpr int ATTN_TILE = 128;      // split boundaries are multiples of this many cached rows
 constexpr int MAX_EVENT_SETS = 256;
-constexpr int SMALL_OUT = 64;       // new rows up to which the last GEMM writes a pageable caller's output to page-locked memory
+// New rows up to which the last GEMM writes a pageable caller's output to page-locked memory.  Its stores
+// cross PCIe before the kernel ends, a copy crosses it at full width but starts behind it: one layer call
+// over 256 cached rows, BASELINE, stores / copy, two boxes: 1 row 110 / 117 us, 16 131 / 133,
+// 25 142 / 148, 32 154 and 162 / 156 and 159, 48 185 and 188 / 183 and 179, 64 223 and 235 / 215 and 217
+// (V4: 1 row 119 / 125, 25 151 / 151, 32 160 and 165 / 159 and 162, 64 229 and 233 / 220).
+constexpr int SMALL_OUT = 32;
 
 struct EventSet {
   cudaEvent_t ev[FST_MLA_K_COUNT + 1];

@@ -271,32 +271,55 @@ def test_plan_is_kept_across_the_layers_of_a_step():
         assert np.array_equal(out0, out3)
 
 
-def test_page_locked_buffers_take_the_direct_paths():
-    """fst_cuda_mla_forward with page-locked, device-addressable buffers (input copied straight from
-    the caller's buffer, output rows written by the last GEMM itself) gives the bits of the same call
-    with pageable buffers (staged copies)."""
+def test_host_buffers_of_every_kind_give_the_bits_of_the_device_call():
+    """fst_cuda_mla_forward with page-locked, device-addressable buffers (input copied straight from the
+    caller's buffer, output rows written by the last GEMM itself), with pageable buffers of up to 32 rows
+    (output written by the last GEMM to page-locked rows of the context) and of more (copied behind the
+    kernels): each gives the bits of fst_cuda_mla_run_device, and the output stage is that of the last
+    call, whatever kind the call before it was."""
     import torch
-    lens, B = [200, 1, 64, 513], 4
-    cfg = mla.make_config(mla.PRESET_BASELINE, n_pages=sum((L + 65) // 64 for L in lens) + 4, max_tokens=B, max_seqs=B)
+    n = 65
+    lens = [(37 * b) % 150 for b in range(n)]
+    cfg = mla.make_config(mla.PRESET_BASELINE, n_pages=sum((L + 65) // 64 for L in lens) + 4, max_tokens=n, max_seqs=n)
     bits, _ = weights_for(mla.PRESET_BASELINE)
     with mla.MlaContext(cfg) as ctx:
         ctx.set_layer_weights(0, bits)
         seqs = []
         for b, L in enumerate(lens):
             s = ctx.seq_alloc()
-            ctx.cache_write(0, s, 0, synth.to_bf16_bits(synth.cache_rows_f32(cfg, 0, b, L)))
+            if L:
+                ctx.cache_write(0, s, 0, synth.to_bf16_bits(synth.cache_rows_f32(cfg, 0, b, L)))
             seqs.append(s)
-        h = synth.to_bf16_bits(synth.hidden_f32(cfg, 0, B, (0,)))
-        ref = ctx.forward(0, h, seqs, lens, [1] * B)
-        for s, L in zip(seqs, lens):
-            ctx.seq_truncate(s, L)
-        h_pin = torch.from_numpy(h.view(np.int16).copy()).pin_memory()
-        out_pin = torch.zeros_like(h_pin).pin_memory()
-        call = ctx.bind_forward(0, h_pin.numpy().view(np.uint16), out_pin.numpy().view(np.uint16),
-                                np.array(seqs, np.int32), np.array(lens, np.int32), np.ones(B, np.int32))
-        call()
-        assert np.array_equal(out_pin.numpy().view(np.uint16), ref)
-        assert np.array_equal(ctx.get_stage(mla.STAGE_OUT), ref)
+        h = synth.to_bf16_bits(synth.hidden_f32(cfg, 0, n, (0,)))
+
+        def rollback(B):
+            for s, L in zip(seqs[:B], lens):
+                ctx.seq_truncate(s, L)
+
+        ref = {}
+        for B in (4, 32, 33, 65):
+            d_h = torch.from_numpy(h[:B].view(np.int16)).cuda()
+            d_out = torch.zeros_like(d_h)
+            torch.cuda.synchronize()
+            ctx.plan([(s, L, 1) for s, L in zip(seqs[:B], lens)])
+            ctx.run_device(0, d_h.data_ptr(), d_out.data_ptr())
+            ctx.sync()
+            ref[B] = d_out.cpu().numpy().view(np.uint16)
+            rollback(B)
+        for B in (4, 32, 33, 65, 32, 65, 4):
+            out = ctx.forward(0, h[:B], seqs[:B], lens[:B], [1] * B)
+            assert np.array_equal(out, ref[B]), B
+            assert np.array_equal(ctx.get_stage(mla.STAGE_OUT), ref[B]), B
+            rollback(B)
+            if B in (32, 65):
+                h_pin = torch.from_numpy(h[:B].view(np.int16).copy()).pin_memory()
+                out_pin = torch.zeros_like(h_pin).pin_memory()
+                call = ctx.bind_forward(0, h_pin.numpy().view(np.uint16), out_pin.numpy().view(np.uint16),
+                                        np.array(seqs[:B], np.int32), np.array(lens[:B], np.int32), np.ones(B, np.int32))
+                call()
+                assert np.array_equal(out_pin.numpy().view(np.uint16), ref[B]), B
+                assert np.array_equal(ctx.get_stage(mla.STAGE_OUT), ref[B]), B
+                rollback(B)
 
 
 def test_forward_with_a_window_set_on_the_context():
