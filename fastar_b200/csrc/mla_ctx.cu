@@ -103,6 +103,22 @@ constexpr int MAX_EVENT_SETS = 256;
 // (V4: 1 row 119 / 125, 25 151 / 151, 32 160 and 165 / 159 and 162, 64 229 and 233 / 220).
 constexpr int SMALL_OUT = 32;
 
+// Page-locked rows with an address on the device, or (false) neither: without them the output is copied
+// behind the kernels.  The three calls are cudaHostAlloc, cudaHostGetDevicePointer and cudaFreeHost, or
+// stand-ins that fail.
+template <class Alloc, class Map, class Free>
+bool mapped_rows(Alloc alloc, Map map, Free release, size_t bytes, void** host, void** dev) {
+  *host = *dev = nullptr;
+  if (alloc(host, bytes) != cudaSuccess) {
+    *host = nullptr;
+    return false;
+  }
+  if (map(dev, *host) == cudaSuccess) return true;
+  release(*host);
+  *host = *dev = nullptr;
+  return false;
+}
+
 struct EventSet {
   cudaEvent_t ev[FST_MLA_K_COUNT + 1];
   bool used[FST_MLA_K_COUNT + 1];
@@ -141,7 +157,7 @@ struct FstMlaCtx {
   bf16* d_cproj = nullptr;       // [T, 2 * width] compressor projections of a call
   uint16_t* h_pinned = nullptr;  // [max_tokens, hidden] staging for the host-buffer entry point
   int* d_status = nullptr;
-  uint16_t* h_out = nullptr;  // [SMALL_OUT, hidden] page-locked output rows of small calls with a pageable h_out
+  uint16_t* h_out = nullptr;  // [SMALL_OUT, hidden] page-locked output rows of small calls with a pageable h_out (null: mapped_rows failed)
   bf16* h_out_dev = nullptr;  // the device's address of it
   const bf16* out_src = nullptr;  // where the last layer call left its output rows
   bool out_zero_copy = true;
@@ -735,9 +751,13 @@ int fst_cuda_mla_create(const FstMlaConfig* cfg, FstMlaCtx** out) {
     cudaGetLastError();
     x->h_status_dev = nullptr;  // no mapping: the status word is copied behind every call instead
   }
-  if (!rc && (cudaHostAlloc((void**)&x->h_out, std::min<size_t>(T, SMALL_OUT) * d.hidden * sizeof(uint16_t), cudaHostAllocMapped) != cudaSuccess ||
-              cudaHostGetDevicePointer((void**)&x->h_out_dev, x->h_out, 0) != cudaSuccess))
-    rc = fail(FST_MLA_ERR_CUDA, "cudaHostAlloc failed");
+  if (!rc) {
+    auto alloc = [](void** p, size_t n) { return cudaHostAlloc(p, n, cudaHostAllocMapped); };
+    auto map = [](void** dev, void* host) { return cudaHostGetDevicePointer(dev, host, 0); };
+    if (!mapped_rows(alloc, map, cudaFreeHost, std::min<size_t>(T, SMALL_OUT) * d.hidden * sizeof(uint16_t), (void**)&x->h_out,
+                     (void**)&x->h_out_dev))
+      cudaGetLastError();
+  }
   if (!rc && cudaHostAlloc((void**)&x->h_pinned, T * d.hidden * sizeof(uint16_t), cudaHostAllocDefault) != cudaSuccess)
     rc = fail(FST_MLA_ERR_CUDA, "cudaHostAlloc failed");
   if (rc) {
@@ -2121,6 +2141,20 @@ int fst_cuda_mla_debug_schedule(int32_t n_sm, const int32_t* pos0, const int32_t
   *n_segs_out = (int)segs.size();
   *n_ctas_out = n_ctas;
   if (cut_by_blocks_out) *cut_by_blocks_out = blocks ? 1 : 0;
+  return FST_MLA_OK;
+}
+
+int fst_cuda_mla_debug_mapped_rows(int32_t alloc_ok, int32_t map_ok, int32_t* host_out, int32_t* device_out, int32_t* held_out) {
+  if (!host_out || !device_out || !held_out) return fail(FST_MLA_ERR_ARG, "null argument");
+  static char row;
+  int held = 0;
+  void *host = nullptr, *dev = nullptr;
+  mapped_rows([&](void** p, size_t) { *p = &row; held += alloc_ok != 0; return alloc_ok ? cudaSuccess : cudaErrorMemoryAllocation; },
+              [&](void** d, void* h) { *d = h; return map_ok ? cudaSuccess : cudaErrorInvalidValue; },
+              [&](void*) { --held; return cudaSuccess; }, sizeof(row), &host, &dev);
+  *host_out = host != nullptr;
+  *device_out = dev != nullptr;
+  *held_out = held;
   return FST_MLA_OK;
 }
 

@@ -140,6 +140,7 @@ def load_library() -> C.CDLL:
     L.fst_cuda_mla_selftest_wait_expiry.argtypes = [vp, i32]
     L.fst_cuda_mla_debug_set_status.argtypes = [vp, i32]
     L.fst_cuda_mla_debug_attr_first_use.argtypes = [C.c_uint64, i32, i64]
+    L.fst_cuda_mla_debug_mapped_rows.argtypes = [i32, i32, i32p, i32p, i32p]
     L.fst_cuda_mla_attention_noalloc.argtypes = [vp, vp, i32, i32, i32, i32, C.c_float, vp, vp]
     _lib = L
     return L

@@ -365,6 +365,13 @@ int fst_cuda_mla_debug_set_status(FstMlaCtx* ctx, int32_t code);
  * (kernel_key, device, value) is seen -- and again when a later value is larger -- else 0. */
 int fst_cuda_mla_debug_attr_first_use(uint64_t kernel_key, int32_t device, int64_t value);
 
+/* Test hook, host only (no CUDA call): page-locked memory that cannot be had, or cannot be mapped, does
+ * not fail fst_cuda_mla_create -- calls of few rows then have their output copied.  Runs that rule
+ * with stand-ins for the allocation and the mapping that succeed or fail as told; reports whether the
+ * context would hold a host and a device address, and how many allocations stay behind. */
+int fst_cuda_mla_debug_mapped_rows(int32_t alloc_ok, int32_t map_ok, int32_t* host_out, int32_t* device_out,
+                                   int32_t* held_out);
+
 /* ---- decode attention without any allocation -------------------------------------------- */
 /* No counterpart in the reference.  For callers that cannot allocate device memory at the
  * moment they need attention: a serving process whose device memory was handed out in full at

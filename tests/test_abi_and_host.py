@@ -51,6 +51,15 @@ def test_bad_config_is_rejected():
     assert b"null" in lib.fst_cuda_mla_last_error()
 
 
+@pytest.mark.parametrize("alloc_ok,map_ok,kept", [(1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 0)])
+def test_output_rows_that_cannot_be_mapped_are_done_without(alloc_ok, map_ok, kept):
+    """A context whose small page-locked output rows cannot be had or mapped holds neither address (the
+    output is then copied) and leaves no allocation behind; it does not refuse to be created."""
+    got = [ctypes.c_int32(-1) for _ in range(3)]
+    assert mla.load_library().fst_cuda_mla_debug_mapped_rows(alloc_ok, map_ok, *(ctypes.byref(x) for x in got)) == 0
+    assert [x.value for x in got] == [kept, kept, kept]
+
+
 def test_bf16_helpers_round_to_nearest_even():
     from oracle import oracle as O
     rng = np.random.default_rng(0)
