@@ -522,6 +522,7 @@ k_gemm_tc_tiles(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
     }
   } else if (warp == 1 && rank == 0) {
+    pdl_wait();  // (the limit of the waits below is for this kernel's own time, not for what is left of the one in front)
     // (warp-uniform walk, one elected lane issues, the next stage's barrier asked ahead: as in k_gemm_tc)
     const uint64_t w_tmpl = W_KN ? tc::umma_desc_sw128(0, W_BYTES / 2, 1024) : tc::umma_desc_sw128(0, 16, 1024);
     const uint64_t a_tmpl = tc::umma_desc_sw128(0, 16, 1024);

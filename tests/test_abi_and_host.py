@@ -60,6 +60,31 @@ def test_output_rows_that_cannot_be_mapped_are_done_without(alloc_ok, map_ok, ke
     assert [x.value for x in got] == [kept, kept, kept]
 
 
+@pytest.mark.parametrize("src,kernel", [("gemm_tc.cu", "k_gemm_tc"), ("gemm_tc.cu", "k_gemm_tc_tiles"),
+                                        ("attn_stream.cu", "k_attn_stream")])
+def test_bounded_waits_start_behind_the_dependency_wait(src, kernel):
+    """These kernels start while the one in front of them still runs.  The limit of their barrier waits is
+    sized for their own work, so in every warp role the first bounded wait has to come behind the wait for
+    the kernel in front.  Read from the source: the roles are the branches on `warp`."""
+    text = open(os.path.join(ROOT, "fastar_b200", "csrc", src)).read()
+    text = re.sub(r"//[^\n]*", "", text)
+    body = text[re.search(r"__global__[^;{]*\b%s\(" % kernel, text).end():]
+    body = body[:body.index("\n}\n")]
+    roles = re.split(r"\n  (?:if \(warp == 0|\} else if \(warp|\} else \{)", body)
+    assert len(roles) >= 4, len(roles)
+    waits = re.compile(r"\b(?:mbar_wait|warp_wait|qk_chunks<[^>]*>)\(")
+    common = "pdl_wait();" in roles[0]
+    assert not waits.search(roles[0])
+    n = 0
+    for role in roles[1:]:
+        first = waits.search(role)
+        if first is None:
+            continue
+        n += 1
+        assert common or 0 <= role.find("pdl_wait();") < first.start(), role[:200]
+    assert n >= 3
+
+
 def test_bf16_helpers_round_to_nearest_even():
     from oracle import oracle as O
     rng = np.random.default_rng(0)
