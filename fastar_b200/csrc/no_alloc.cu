@@ -25,6 +25,8 @@ constexpr int NA_MAX_DV = 512;
 constexpr int NA_MAX_DQK = 576;
 constexpr int NA_MAX_SPLITS = 148;   // KV splits = thread blocks of the attention kernel: one per SM
 constexpr int NA_PAGE = 64;
+constexpr int NA_SIMT_SPLITS = 32;   // the same of the CUDA-core kernel (the only ones with a segment in memory)
+constexpr int NA_SIMT_UNIT = 32;     // its rows per schedule tile
 constexpr int NA_MIN_SPLITS = 32;    // blocks that a cache is spread over before one takes a second page
 constexpr int NA_PAGES_PER_BLOCK = 2;
 
@@ -35,9 +37,10 @@ constexpr size_t OFF_PART_M = OFF_PART_O + SZ_PART_O;
 constexpr size_t SZ_PART_ML = (size_t)NA_MAX_SPLITS * NA_MAX_HEADS * sizeof(float);
 constexpr size_t OFF_PART_L = OFF_PART_M + SZ_PART_ML;
 constexpr size_t OFF_SEGS = OFF_PART_L + SZ_PART_ML;
-constexpr size_t OFF_TABLE = OFF_SEGS + 3072;                                   // 148 segments x 20 bytes, padded
+constexpr size_t OFF_TABLE = OFF_SEGS + 1024;                                   // NA_SIMT_SPLITS segments x 20 bytes, padded
 constexpr size_t OFF_TOK = OFF_TABLE + (NA_MAX_ROWS / NA_PAGE) * sizeof(int32_t);  // tok_table[1], tok_part[2];
-                                                                                // int 60: status
+                                                                                // int 60: what a wait that ran
+                                                                                // out records; nothing reads it
 constexpr size_t OFF_LUT = OFF_TOK + 256;                                       // unused RoPE table slot
 constexpr size_t SCRATCH_BYTES = OFF_LUT + 256;
 
@@ -52,8 +55,7 @@ unsigned char* g_na_ptr[64] = {nullptr};
 // Rewrites every piece of bookkeeping the CUDA-core attention kernel and its merge read from the
 // scratch: an identity block table (the cache is contiguous), the split schedule, the one-token
 // maps.  (The tcgen05 kernel works its run out from the block index: AttnArgs::flat_rows.)
-// unit: rows per schedule tile.
-__global__ void k_na_setup(unsigned char* scratch, int n_rows, int n_splits, int unit) {
+__global__ void k_na_setup(unsigned char* scratch, int n_rows, int n_splits) {
   AttnSeg* segs = reinterpret_cast<AttnSeg*>(scratch + OFF_SEGS);
   int32_t* table = reinterpret_cast<int32_t*>(scratch + OFF_TABLE);
   int32_t* tok = reinterpret_cast<int32_t*>(scratch + OFF_TOK);
@@ -61,12 +63,12 @@ __global__ void k_na_setup(unsigned char* scratch, int n_rows, int n_splits, int
   for (int i = threadIdx.x; i < n_pages; i += blockDim.x) table[i] = i;
   if (threadIdx.x < n_splits) {
     // equal runs of tiles; the last split takes the ragged end
-    const int tiles = (n_rows + unit - 1) / unit;
+    const int tiles = (n_rows + NA_SIMT_UNIT - 1) / NA_SIMT_UNIT;
     const int s = threadIdx.x;
     AttnSeg sg;
     sg.tok = 0;
-    sg.kv_begin = (int)((long long)tiles * s / n_splits) * unit;
-    sg.kv_end = min(n_rows, (int)((long long)tiles * (s + 1) / n_splits) * unit);
+    sg.kv_begin = (int)((long long)tiles * s / n_splits) * NA_SIMT_UNIT;
+    sg.kv_end = min(n_rows, (int)((long long)tiles * (s + 1) / n_splits) * NA_SIMT_UNIT);
     sg.part = s;
     sg.table = 0;  // the identity block table starts at entry 0
     segs[s] = sg;
@@ -143,7 +145,7 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   a.scale = softmax_scale;
   // The full MLA shape (64 heads, 576- or 512-wide rows, 512 value columns) goes to the tcgen05
   // streaming kernel, one thread block per run of whole 64-row pages; every other shape to the
-  // CUDA-core kernel (so do caches of less than one page) on at most 32 blocks.
+  // CUDA-core kernel (so do caches of less than one page) on at most NA_SIMT_SPLITS blocks.
   // A block streams about 40 bytes per clock, so the pages are spread over every SM -- but from 64 pages
   // on no thinner than NA_PAGES_PER_BLOCK pages each: every block leaves 128 KB of partials behind.  With
   // 32 blocks and the schedule written by a kernel in front 20 000 rows took 32.8 us, now 26.0.
@@ -155,7 +157,7 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
   const int n_pages = (n_rows + NA_PAGE - 1) / NA_PAGE;
   const int n_splits = stream ? std::max(std::min(NA_MIN_SPLITS, n_pages),
                                          std::min(NA_MAX_SPLITS, (n_pages + NA_PAGES_PER_BLOCK - 1) / NA_PAGES_PER_BLOCK))
-                              : std::max(1, std::min(32, (n_rows + 127) / 128));
+                              : std::max(1, std::min(NA_SIMT_SPLITS, (n_rows + 127) / 128));
   a.n_segs = n_splits;
   a.n_ctas = n_splits;
   if (stream) {
@@ -164,7 +166,7 @@ extern "C" int fst_cuda_mla_attention_noalloc(const void* d_q_eff, const void* d
     cudaError_t es = launch_attn_stream(a, st);
     if (es != cudaSuccess) return na_fail(FST_MLA_ERR_CUDA, cudaGetErrorString(es));
   } else {
-    k_na_setup<<<1, 256, 0, st>>>(sc, n_rows, n_splits, 32);
+    k_na_setup<<<1, 256, 0, st>>>(sc, n_rows, n_splits);
     launch_attn_simt(a, st);
   }
 
