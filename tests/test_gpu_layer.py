@@ -28,15 +28,22 @@ def weights_for(preset, attn_norm=False):
 
 
 def run_layer(preset, impl, lens, q_len, causal, seed=0, steps=1, ulps=0, attn_norm=False, rope_yarn=False,
-              yarn_by_layer_call=False):
-    """`steps` consecutive layer calls (each appends q_len tokens per sequence); every call is
-    compared with the oracle, and so is the cache content afterwards."""
+              yarn_by_layer_call=False, sizes=None):
+    """`steps` consecutive layer calls (each appends q_len tokens per sequence, or q_len[b] to sequence
+    b); every call is compared with the oracle, and so is the cache content afterwards.  sizes:
+    configuration values other than the preset's."""
     attn_impl, gemm_impl = impl[1], impl[2]
     B = len(lens)
-    n_pages = sum((L + q_len * steps + 63) // 64 for L in lens) + 4
-    cfg = mla.make_config(preset, n_pages=n_pages, max_tokens=B * q_len, max_seqs=B, attn_impl=attn_impl,
-                          gemm_impl=gemm_impl, rope_yarn=rope_yarn and not yarn_by_layer_call)
-    bits, rounded = weights_for(preset, attn_norm)
+    q_lens = [q_len] * B if isinstance(q_len, int) else list(q_len)
+    T = sum(q_lens)
+    n_pages = sum((L + q * steps + 63) // 64 for L, q in zip(lens, q_lens)) + 4
+    cfg = mla.make_config(preset, n_pages=n_pages, max_tokens=T, max_seqs=B, attn_impl=attn_impl,
+                          gemm_impl=gemm_impl, rope_yarn=rope_yarn and not yarn_by_layer_call, **(sizes or {}))
+    if sizes:
+        w = synth.layer_weights_f32(cfg, 0, 0)
+        bits, rounded = synth.weights_to_bits(w), synth.weights_rounded(w)
+    else:
+        bits, rounded = weights_for(preset, attn_norm)
     ocfg = oracle_cfg(cfg)
     ocfg.rope_yarn = int(rope_yarn)
     d = mla.dims_of(cfg)
@@ -52,21 +59,21 @@ def run_layer(preset, impl, lens, q_len, causal, seed=0, steps=1, ulps=0, attn_n
             if L:
                 ctx.cache_write(0, s, 0, rows)
             seqs.append(s)
-            cache = np.zeros((L + q_len * steps, d["row"]), np.float32)
+            cache = np.zeros((L + q_lens[b] * steps, d["row"]), np.float32)
             cache[:L] = synth.from_bf16_bits(rows)
             caches.append(cache)
         pos = list(lens)
         for step in range(steps):
-            h = synth.to_bf16_bits(synth.hidden_f32(cfg, seed, B * q_len, (step,)))
-            out = ctx.forward(0, h, seqs, pos, [q_len] * B, causal=causal)
+            h = synth.to_bf16_bits(synth.hidden_f32(cfg, seed, T, (step,)))
+            out = ctx.forward(0, h, seqs, pos, q_lens, causal=causal)
             stages = {k: ctx.get_stage(v) for k, v in (("qc", mla.STAGE_QC), ("kv", mla.STAGE_KV),
                                                       ("q_eff", mla.STAGE_QEFF), ("o_lat", mla.STAGE_OLAT),
                                                       ("low", mla.STAGE_LOW))}
             hf = synth.from_bf16_bits(h)
             for b in range(B):
-                r = O.mla_forward(ocfg, rounded, hf[b * q_len:(b + 1) * q_len], pos[b], caches[b], causal=causal)
-                sl = slice(b * q_len, (b + 1) * q_len)
-                slh = slice(b * q_len * H, (b + 1) * q_len * H)
+                sl = slice(sum(q_lens[:b]), sum(q_lens[:b + 1]))
+                slh = slice(sl.start * H, sl.stop * H)
+                r = O.mla_forward(ocfg, rounded, hf[sl], pos[b], caches[b], causal=causal)
                 # normed intermediates are O(1..8): one or two bf16 steps there exceed 2e-2
                 check_close(stages["qc"][sl], r.trace["qc"], f"step {step} seq {b} qc", ulps=2)
                 check_close(stages["kv"][sl], r.trace["kv"], f"step {step} seq {b} kv", ulps=2)
@@ -76,9 +83,9 @@ def run_layer(preset, impl, lens, q_len, causal, seed=0, steps=1, ulps=0, attn_n
                 check_close(out[sl], r.out, f"step {step} seq {b} out", ulps=ulps)
                 # cache push: the appended rows are the kv stage rows, bit for bit, at the rows
                 # the block table names
-                got_rows = ctx.cache_read(0, seqs[b], pos[b], q_len)
+                got_rows = ctx.cache_read(0, seqs[b], pos[b], q_lens[b])
                 assert np.array_equal(got_rows, stages["kv"][sl])
-                pos[b] += q_len
+                pos[b] += q_lens[b]
         # the history itself is untouched
         for b, L in enumerate(lens):
             if L:
@@ -166,6 +173,23 @@ def test_attn_norm_in_front_of_the_layer(impl, preset):
     # before attn_norm and applies it itself; inputs with a row scale far from 1 so that a missing
     # norm cannot pass
     run_layer(preset, impl, [300, 65], 2, True, seed=5, steps=2, ulps=2, attn_norm=True)
+
+
+@pytest.mark.parametrize("preset", [mla.PRESET_BASELINE, mla.PRESET_FASTAR_V4], ids=["baseline", "v4"])
+@pytest.mark.parametrize("lens,q_lens", [([70], [129]), ([200, 0], [161, 140]), ([5, 130, 0], [43, 97, 60])],
+                         ids=["129", "301", "200"])
+def test_ragged_prompts_of_more_than_128_tokens(preset, lens, q_lens):
+    """What runs above 128 tokens, stage by stage: the persistent GEMM (batch members as the middle
+    tensor-map coordinate, strided outputs, the q_pe rotation on its epilogue warps) and the 256-token tile
+    with a K split, last token tiles of 1 and 45 tokens, two query rows per warp in the V4 head norm,
+    attn_norm in front (V4)."""
+    run_layer(preset, IMPLS[1], lens, q_lens, True, seed=8, ulps=2, attn_norm=preset == mla.PRESET_FASTAR_V4)
+
+
+def test_an_odd_number_of_query_rows_in_the_head_norm():
+    # 249 tokens x 33 heads: 8217 rows, two to a warp, the last warp with one
+    run_layer(mla.PRESET_FASTAR_V4, ("auto", mla.IMPL_AUTO, mla.IMPL_AUTO), [20], 249, True, seed=9, ulps=2,
+              sizes=dict(hidden=512, n_heads=33, q_lora=128, o_lora=128))
 
 
 @pytest.mark.parametrize("impl", IMPLS, ids=[i[0] for i in IMPLS])

@@ -56,9 +56,12 @@ def test_matches_the_regular_entry_point_twice_in_a_row():
 
 
 @pytest.mark.parametrize("heads,d_qk,d_v,n_rows", [(64, 576, 512, 1), (64, 576, 512, 129), (5, 72, 64, 300),
-                                                   (16, 512, 512, 1000), (3, 136, 128, 33)])
+                                                   (16, 512, 512, 1000), (3, 136, 128, 33)] +
+                         # the tcgen05 kernel: one page and its edge, two pages, the row counts around which the rule for
+                         # the number of blocks changes (32, 64 and 296 pages)
+                         [(64, w, 512, n) for w in (576, 512) for n in (64, 65, 128, 129, 2048, 2049, 4096, 4097, 18944, 18945)])
 def test_small_and_odd_shapes_against_the_cpu_oracle(heads, d_qk, d_v, n_rows):
-    """Fewer than 64 heads, narrow rows, one row, a ragged second split: each against the oracle's
+    """Fewer than 64 heads, narrow rows, one row, a ragged second split, the full shape in both widths: each against the oracle's
     attention on the same bits (rows are d_qk wide with no padding; values are row[:d_v])."""
     rng = np.random.default_rng(heads * 1000 + n_rows)
     rows = synth.to_bf16_bits(rng.standard_normal((n_rows, d_qk)).astype(np.float32))
