@@ -1557,8 +1557,12 @@ int plan_schedule_part(FstMlaCtx* c, bool on_copy_stream) {
       S.n_single_part += np == 1;
     }
     // Tiles come from L2 when the lanes of a group read them side by side, and when all rows that the
-    // call attends to stay resident (at most half of L2) and are read several times over, as a prompt
-    // does (2048 tokens: attention 427 -> 389 us, alone).
+    // call attends to stay resident (at most 64 MiB, about half of the L2) and are read several times over,
+    // as a prompt does (2048 tokens: attention 427 -> 389 us, alone).  Layer calls without /
+    // with it: 3 prompts of 100-150 rows behind 300 171 / 166 us, 2 of 150-200 behind 1000 204 / 196 (V4
+    // 232 / 225), 1300 rows 477 / 467 (V4 605 / 602), 12 blocks of 9-14 behind 1200 131 / 128; with fewer
+    // than ten tiles per block (verify blocks of 5 to 16 rows over some hundred) within what two
+    // processes of one build differ by.
     long long rows_once = 0;
     for (const FstMlaSeqStep& step : c->pl_steps)
       if (step.q_len > 0) rows_once += step.append ? step.pos0 + step.q_len : step.pos0;
