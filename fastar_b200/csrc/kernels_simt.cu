@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(256) k_norm_append(NormAppendArgs a) {
 
 // The same with 16 bytes (eight elements) per thread: the first warps take the query row, the others
 // the key row.  RoPE pairs never leave their thread, so one block barrier (the sums of squares) is
-// left of three.  One row 5.8 -> 3.7 us, 2048 rows 15.7 -> 7.8 us (each alone).  Nothing is loaded before
+// left of three.  One row 5.8 -> 3.3-4.5 us, 2048 rows 15.7 -> 7.8 us (each alone).  Nothing is loaded before
 // the wait, although weights, RoPE row and destination could be.  Layer calls with these loads beside the
 // GEMM in front, against the scalar kernel and against this one: BASELINE, one row over 131 072 rows 105.2
 // (scalar 102.5) on one box, 100.3 (this one 100.1; scalar 101.1) on others; V4, five tokens, two layers
