@@ -44,7 +44,9 @@ constexpr size_t OFF_TOK = OFF_TABLE + (NA_MAX_ROWS / NA_PAGE) * sizeof(int32_t)
 constexpr size_t OFF_LUT = OFF_TOK + 256;                                       // unused RoPE table slot
 constexpr size_t SCRATCH_BYTES = OFF_LUT + 256;
 
-// Every GPU that loads the library holds this array (about 18.6 MiB) until the process exits.
+// About 18.6 MiB.  CUDA loads this file's code, and with it the array, at the first call on a device (free
+// memory there fell by 20 MiB with it, by nothing with the library's loading or a context's creation),
+// and holds it until the process exits.
 static __device__ __align__(256) unsigned char g_na_scratch[SCRATCH_BYTES];
 
 // Device address of g_na_scratch per device.  In host code the array's name is only a

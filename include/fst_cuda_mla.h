@@ -385,8 +385,11 @@ int fst_cuda_mla_debug_mapped_rows(int32_t alloc_ok, int32_t map_ok, int32_t* ho
  * = softmax(scale * q K^T) V, no sink.  Both inputs 16-byte aligned.  Work is enqueued on
  * cuda_stream (NULL: default stream) of the current device; the call does not synchronise.
  *
- * The split-KV partials live in a fixed array inside the library image (about 18.6 MiB, held by
- * every GPU that loads the library until the process exits), hence the limits: n_rows <= 65536,
+ * The split-KV partials live in a fixed array inside the library image (about 18.6 MiB, part of
+ * its GPU code: the driver places it on a GPU with the first call there -- at start-up with
+ * CUDA_MODULE_LOADING=EAGER -- and holds it until the process exits; a process that makes no such
+ * call holds nothing of it, one that budgets its memory makes a first call before handing the rest
+ * out), hence the limits: n_rows <= 65536,
  * n_heads <= 64, d_qk <= 576 (multiple of 8), d_v <= 512 (multiple of 64, <= d_qk).  Anything
  * larger returns FST_MLA_ERR_CAPACITY (fst_cuda_mla_last_error says why); use the context API
  * then.  A CUDA error that an earlier call left pending on the calling thread is reported as
