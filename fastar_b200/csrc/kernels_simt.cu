@@ -283,14 +283,16 @@ __global__ void __launch_bounds__(256) k_norm_append(NormAppendArgs a) {
 
 // The same with 16 bytes (eight elements) per thread: the first warps take the query row, the others
 // the key row.  RoPE pairs never leave their thread, so one block barrier (the sums of squares) is
-// left of three.  One row 5.8 -> 3.3-4.5 us, 2048 rows 15.7 -> 7.8 us (each alone).  Nothing is loaded before
-// the wait, although weights, RoPE row and destination could be.  Layer calls with these loads beside the
-// GEMM in front, against the scalar kernel and against this one: BASELINE, one row over 131 072 rows 105.2
-// (scalar 102.5) on one box, 100.3 (this one 100.1; scalar 101.1) on others; V4, five tokens, two layers
-// 209.0 (210.3).  What one form loses there is more than the other gains.
+// left of three.  One row 5.8 -> 3.3-4.5 us, 2048 rows 15.7 -> 7.8 us (each alone).  Weights, RoPE row and
+// destination are the layer's or the plan's and could all be read before the wait; that pays for rows without
+// a part of their own for RoPE (V4) and costs with one (BASELINE), by measurement alone.  Layer calls with the
+// early reads / without, us: V4 two layers of 5 users 210.1 / 212.3, of 2 users 158.4 / 159.6, of one 224.2 /
+// 227.2; BASELINE one row over 131 072 rows 102.4 / 101.8 (on another box 105.2, where the scalar kernel took
+// 102.5), over 4096 74.5 / 74.4.
 __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
   pdl_launch();
-  pdl_wait();
+  const bool early = a.row == a.kv_lora;
+  if (!early) pdl_wait();
   __shared__ float scratch[32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int q_warps = (a.q_lora / 8 + 31) / 32;  // the rest of the block has the key row
@@ -309,6 +311,7 @@ __global__ void __launch_bounds__(512) k_norm_append_vec(NormAppendArgs a) {
     l1 = lut[1];
   }
   const long long dst = a.dst_row[t];
+  if (early) pdl_wait();
   const bf16* in = a.cmp + (long long)t * (a.q_lora + a.row) + (is_q ? 0 : a.q_lora);
   if (on) xv = *reinterpret_cast<const uint4*>(in + j0);
   float x[8];
